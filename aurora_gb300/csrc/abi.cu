@@ -59,6 +59,11 @@ cudaError_t alloc_device_async(void** p, size_t bytes, cudaStream_t s) {
     return cudaMallocAsync(p, bytes, s);
 }
 
+cudaError_t alloc_device_pool(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t s) {
+    if (injected_failure()) { *p = nullptr; return cudaErrorMemoryAllocation; }
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
 cudaError_t alloc_pinned(void** p, size_t bytes) {
     if (injected_failure()) { *p = nullptr; return cudaErrorMemoryAllocation; }
     return cudaHostAlloc(p, bytes, cudaHostAllocDefault);
@@ -150,6 +155,7 @@ aur_status aur_ctx_create(int device, aur_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->compute2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = ::aur::dev_malloc(&c->d_flags, 256);
     if (e == cudaSuccess) e = cudaMemset(c->d_flags, 0, 256);
+    if (e == cudaSuccess) e = ::aur::create_nmh_pool(device, &c->nmh_pool);
     if (e != cudaSuccess) {
         cudaGetLastError();
         aur_ctx_destroy(c);
@@ -234,11 +240,9 @@ aur_status aur_nmh_build(aur_ctx* ctx, const float* vertices, uint32_t count, au
 aur_status aur_nmh_destroy(aur_nmh* nmh) {
     if (!nmh) return AUR_OK;
     cudaSetDevice(nmh->device);
-    if (nmh->rec_tex) {
-        cudaDeviceSynchronize();   // no traversal may still read through the texture
-        cudaDestroyTextureObject(nmh->rec_tex);
-    }
-    cudaFree(nmh->mem);
+    cudaDeviceSynchronize();   // no launch may still read it
+    if (nmh->rec_tex) cudaDestroyTextureObject(nmh->rec_tex);
+    if (nmh->mem && cudaFreeAsync(nmh->mem, cudaStreamLegacy) != cudaSuccess) cudaGetLastError();
     delete nmh;
     return AUR_OK;
 }

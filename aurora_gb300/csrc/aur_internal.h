@@ -4,6 +4,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <memory>
 
 #include "../../include/aurora_gb300.h"
 
@@ -30,6 +31,7 @@ void clear_error();
 // each caller's out-of-memory path.
 cudaError_t alloc_device(void** p, size_t bytes);
 cudaError_t alloc_device_async(void** p, size_t bytes, cudaStream_t s);
+cudaError_t alloc_device_pool(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t s);
 cudaError_t alloc_pinned(void** p, size_t bytes);
 template <typename T>
 inline cudaError_t dev_malloc(T** p, size_t bytes) { return alloc_device((void**)p, bytes); }
@@ -61,6 +63,14 @@ constexpr int kStackDepth = 32;
 // by nmh_build.cu; freed with the context.
 struct BuildCache;
 
+// The pool that NMH memory comes from. Shared by a context and the NMHs built
+// on it, which may outlive the context: the last of them destroys it.
+struct NmhPool {
+    int device = 0;
+    cudaMemPool_t pool = nullptr;
+    ~NmhPool();
+};
+
 }  // namespace aur
 
 struct aur_ctx {
@@ -76,6 +86,7 @@ struct aur_ctx {
     aur::Scratch out[2];
     aur::Scratch defer[2];               // per trace slot: ray chunks left to the per-lane kernel
     cudaEvent_t ev[8] = {};
+    std::shared_ptr<aur::NmhPool> nmh_pool;   // memory of the NMHs built on this context
     aur::BuildCache* build = nullptr;    // created by the first aur_nmh_build
     uint32_t lookback_test = 0;          // test hook for the next build (aur_debug_lookback_timeout)
 };
@@ -86,7 +97,8 @@ struct aur_nmh {
     uint32_t input_count = 0; // triangles as given
     uint32_t levels = 0;
     uint32_t nodes = 0;       // count / 2
-    void* mem = nullptr;          // one allocation holding the three arrays below
+    std::shared_ptr<aur::NmhPool> pool;
+    void* mem = nullptr;          // from the pool: one allocation holding the three arrays below
     float4* node_recs = nullptr;  // nodes * 8 float4 (slab, 2 x (v1, e1, e2), children's boxes)
     uint32_t* perm = nullptr;     // NMH position -> original prim id
     float* verts = nullptr;       // count * 9, NMH order, reference layout
@@ -124,6 +136,7 @@ struct aur_scene {
 
 namespace aur {
 
+cudaError_t create_nmh_pool(int device, std::shared_ptr<NmhPool>* out);
 aur_status nmh_build_impl(aur_ctx* ctx, const float* vertices, uint32_t count, aur_nmh** out);
 // Releases the context's cached build scratch and graph (after its last launch).
 void free_build_cache(aur_ctx* ctx);

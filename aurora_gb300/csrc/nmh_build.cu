@@ -1442,6 +1442,36 @@ static float record_extent(const float* r, uint32_t nodes) {
     return std::isfinite(e) ? e : 0.0f;
 }
 
+// NMH memory comes from a pool of the context, allocated and freed in stream
+// order: a plain cudaMalloc / cudaFree pair maps and unmaps device memory for
+// every NMH over 2 MB, which is most of a small rebuild's time. The pool keeps
+// at most kNmhPoolBytes of freed memory (a 1M-triangle NMH, rebuilt every
+// frame, takes 121 MB) and gives back what is above that at the next
+// synchronization, all of it with the context and its last NMH.
+constexpr uint64_t kNmhPoolBytes = 256ull << 20;
+
+NmhPool::~NmhPool() {
+    if (!pool) return;
+    cudaSetDevice(device);
+    cudaStreamSynchronize(cudaStreamLegacy);   // the last NMH was freed there
+    cudaMemPoolDestroy(pool);
+}
+
+cudaError_t create_nmh_pool(int device, std::shared_ptr<NmhPool>* out) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    auto p = std::make_shared<NmhPool>();
+    p->device = device;
+    cudaError_t e = cudaMemPoolCreate(&p->pool, &props);
+    uint64_t keep = kNmhPoolBytes;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess) *out = std::move(p);
+    return e;
+}
+
 aur_status nmh_build_impl(aur_ctx* ctx, const float* V, uint32_t count, aur_nmh** out) {
     AUR_CHECK(ctx && out, AUR_ERR_INVALID, "aur_nmh_build: null context or output pointer");
     AUR_CHECK(count == 0 || V, AUR_ERR_INVALID, "aur_nmh_build: null vertices for %u triangles", count);
@@ -1452,20 +1482,27 @@ aur_status nmh_build_impl(aur_ctx* ctx, const float* V, uint32_t count, aur_nmh*
     const uint32_t n = N / 2;
     aur_nmh* nmh = new aur_nmh();
     nmh->device = ctx->device;
+    nmh->pool = ctx->nmh_pool;
     nmh->count = N;
     nmh->input_count = count;
     nmh->nodes = n;
     nmh->levels = n ? log2i(n) + 1 : 0;
     if (N == 0) { *out = nmh; return AUR_OK; }
 
+    cudaStream_t st = ctx->stream;
     auto cleanup = [&]() {
-        cudaFree(nmh->mem);
+        if (nmh->mem) {
+            cudaStreamSynchronize(st);
+            cudaFreeAsync(nmh->mem, cudaStreamLegacy);
+        }
         delete nmh;
     };
     // records, permutation and vertices in one allocation (records first: 128-byte aligned)
     const size_t b_recs = ((size_t)n * kRecStride * sizeof(float4) + 255) & ~(size_t)255;
     const size_t b_perm = ((size_t)N * sizeof(uint32_t) + 255) & ~(size_t)255;
-    if (::aur::dev_malloc(&nmh->mem, b_recs + b_perm + (size_t)N * 9 * sizeof(float)) != cudaSuccess) {
+    if (::aur::alloc_device_pool(&nmh->mem, b_recs + b_perm + (size_t)N * 9 * sizeof(float), ctx->nmh_pool->pool, st) !=
+        cudaSuccess) {
+        nmh->mem = nullptr;
         cudaGetLastError();
         cleanup();
         return fail(AUR_ERR_OOM, "aur_nmh_build: out of device memory for %u triangles", N);
@@ -1474,7 +1511,6 @@ aur_status nmh_build_impl(aur_ctx* ctx, const float* V, uint32_t count, aur_nmh*
     nmh->perm = (uint32_t*)((char*)nmh->mem + b_recs);
     nmh->verts = (float*)((char*)nmh->mem + b_recs + b_perm);
 
-    cudaStream_t st = ctx->stream;
     BuildArgs a{V, count, nmh->node_recs, nmh->perm, nmh->verts, nullptr, ctx->d_flags};
     a.lookback_test = ctx->lookback_test;     // armed for this one build only
     ctx->lookback_test = 0;
