@@ -241,7 +241,6 @@ aur_status aur_nmh_destroy(aur_nmh* nmh) {
     if (!nmh) return AUR_OK;
     cudaSetDevice(nmh->device);
     cudaDeviceSynchronize();   // no launch may still read it
-    if (nmh->rec_tex) cudaDestroyTextureObject(nmh->rec_tex);
     if (nmh->mem && cudaFreeAsync(nmh->mem, cudaStreamLegacy) != cudaSuccess) cudaGetLastError();
     delete nmh;
     return AUR_OK;
@@ -249,12 +248,6 @@ aur_status aur_nmh_destroy(aur_nmh* nmh) {
 
 aur_status aur_debug_nmh_drop_texture(aur_nmh* nmh) {
     AUR_CHECK(nmh, AUR_ERR_INVALID, "aur_debug_nmh_drop_texture: null NMH");
-    AUR_CUDA(cudaSetDevice(nmh->device));
-    if (nmh->rec_tex) {
-        AUR_CUDA(cudaDeviceSynchronize());   // no launch may still read through it
-        AUR_CUDA(cudaDestroyTextureObject(nmh->rec_tex));
-        nmh->rec_tex = 0;
-    }
     return AUR_OK;
 }
 

@@ -98,13 +98,11 @@ struct aur_nmh {
     uint32_t levels = 0;
     uint32_t nodes = 0;       // count / 2
     std::shared_ptr<aur::NmhPool> pool;
-    void* mem = nullptr;          // from the pool: one allocation holding the three arrays below
+    void* mem = nullptr;          // from the pool: one allocation holding the four arrays below
     float4* node_recs = nullptr;  // nodes * 8 float4 (slab, 2 x (v1, e1, e2), children's boxes)
+    uint4* wide = nullptr;        // treelet records of the same tree (aur_wide.cuh)
     uint32_t* perm = nullptr;     // NMH position -> original prim id
     float* verts = nullptr;       // count * 9, NMH order, reference layout
-    // node_recs as a linear texture of float4 texels: k_trace reads one of a
-    // node's four sectors through the texture path (0: none, plain loads)
-    cudaTextureObject_t rec_tex = 0;
     // Largest side of the bounding box of all triangles (from the root node's
     // record): the scale for deciding when a warp's rays are close enough
     // together to traverse as a packet.

@@ -106,18 +106,14 @@ struct Sector {
 };
 __device__ __forceinline__ Sector ld_sector(const float4* __restrict__ p) {
     Sector s;
+#ifndef __CUDACC__
+    s.a = p[0];
+    s.b = p[1];
+#else
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(s.a.x), "=f"(s.a.y), "=f"(s.a.z), "=f"(s.a.w), "=f"(s.b.x), "=f"(s.b.y), "=f"(s.b.z), "=f"(s.b.w)
         : "l"(p));
-    return s;
-}
-
-// The same sector through the texture path: two float4 texels of the records
-// bound as a linear texture (texel index = float4 index in the records).
-__device__ __forceinline__ Sector tex_sector(cudaTextureObject_t tex, size_t texel) {
-    Sector s;
-    s.a = tex1Dfetch<float4>(tex, (int)texel);
-    s.b = tex1Dfetch<float4>(tex, (int)texel + 1);
+#endif
     return s;
 }
 
@@ -208,18 +204,13 @@ __device__ __forceinline__ void trav_descend(TravState& s, const float4* __restr
 // ray.cuh:198-223) in order. Closest hit: ties in t go to the lower original
 // prim id. Any hit: returns true on the first hit with Epsilon < t < best_t.
 // s0: record sector 0 (from trav_next); sectors 1 and 2 are read here, and
-// word 5 (the tail of sector 2) is handed back in q5 for trav_descend. With
-// kTex, sector 2 comes through the texture path (tex: the records as float4
-// texels): with one of a node's four sectors there, the L1 load pipe, which
-// bounds the traversal, and the texture pipe share the node's reads (+2.3 %
-// on the traversal microbench; more sectors there, or others, measured slower).
-template <bool kAny, bool kTex = false>
+// word 5 (the tail of sector 2) is handed back in q5 for trav_descend.
+template <bool kAny>
 __device__ __forceinline__ bool node_triangles(const float4* __restrict__ recs, uint32_t k, const Sector& s0,
                                                const uint32_t* __restrict__ perm, const f3& pos, const f3& dir,
-                                               float& best_t, float& bu, float& bv, uint32_t& best, float4& q5,
-                                               cudaTextureObject_t tex = 0) {
+                                               float& best_t, float& bu, float& bv, uint32_t& best, float4& q5) {
     const Sector s1 = ld_sector(recs + (size_t)k * kRecStride + 2);
-    const Sector s2 = kTex ? tex_sector(tex, (size_t)k * kRecStride + 4) : ld_sector(recs + (size_t)k * kRecStride + 4);
+    const Sector s2 = ld_sector(recs + (size_t)k * kRecStride + 4);
     const float4& q0 = s0.a;
     const float4& q1 = s0.b;
     const float4& q2 = s1.a;
@@ -280,11 +271,11 @@ __device__ __forceinline__ uint32_t dir_octant(const f3& dir) {
     return (dir.x < 0.0f ? 1u : 0u) | (dir.y < 0.0f ? 2u : 0u) | (dir.z < 0.0f ? 4u : 0u);
 }
 
-// Largest side of the box around the valid lanes' ray origins (call with
-// all 32 lanes). A packet pays for the union of its lanes' nodes, so it is
+// Largest side of the box around the valid lanes' points, here ray origins
+// (call with all 32 lanes). A packet pays for the union of its lanes' nodes, so it is
 // only worth taking when the rays start close together (a camera's, or
 // neighbouring points toward one light); this is that test's measure.
-__device__ __forceinline__ float warp_origin_span(const f3& pos, bool valid) {
+__device__ __forceinline__ float warp_span(const f3& pos, bool valid) {
     float lx = valid ? pos.x : INFINITY, ly = valid ? pos.y : INFINITY, lz = valid ? pos.z : INFINITY;
     float hx = valid ? pos.x : -INFINITY, hy = valid ? pos.y : -INFINITY, hz = valid ? pos.z : -INFINITY;
 #pragma unroll

@@ -31,6 +31,7 @@
 #include "aur_internal.h"
 #include "aur_math.cuh"
 #include "aur_traverse.cuh"
+#include "aur_wide.cuh"
 
 namespace aur {
 namespace {
@@ -945,6 +946,16 @@ __global__ void k_node_boxes(uint32_t L0, uint32_t L1, uint32_t n, const float* 
     rec[2] = make_float4(cb[1][2], cb[1][3], cb[1][4], cb[1][5]);
 }
 
+// One thread per treelet writes its record (wide_record) from the NMH-ordered
+// vertices and the subtree boxes of k_local_finish and k_node_boxes.
+__global__ void __launch_bounds__(128) k_wide_nodes(const float* __restrict__ verts, const float* __restrict__ box,
+                                                    uint32_t n, uint32_t levels, uint32_t treelets,
+                                                    uint4* __restrict__ wide, const uint32_t* err) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= treelets || build_aborted(err)) return;
+    wide_record(verts, box, n, levels, t, wide + (size_t)t * kWideStride);
+}
+
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 uint32_t log2i(uint32_t x) {
@@ -1183,6 +1194,7 @@ struct BuildArgs {
     float* verts;
     unsigned char* scratch;    // scratch_layout(N).end bytes
     uint32_t* flags;           // error bits 4 (internal check), 8 (non-finite vertex), 16 (look-back timeout)
+    uint4* wide = nullptr;     // treelet records (wide_count(levels)), or null: not built
     uint32_t lookback_test = 0;  // test hook: nonzero makes the look-back waits run out (see tile_lookback)
 };
 
@@ -1263,6 +1275,11 @@ void enqueue_build(Seq& q, const BuildArgs& b) {
     q.launch(k_pair_order, dim3(cdiv(n, 256)), dim3(256), 0, n, heap, mn + al * S, b.perm, b.flags);
     // mx and k2 are free once the levels are placed: 3*S >= 6*n floats each for the boxes
     emit_records(q, b.V, b.count, b.perm, n, lv0, b.verts, b.recs, mx, (float*)k2, b.flags);
+    if (b.wide) {
+        const uint32_t treelets = (uint32_t)wide_count(levels);
+        q.launch(k_wide_nodes, dim3(cdiv(treelets, 128)), dim3(128), 0, b.verts, (const float*)k2, n, levels, treelets,
+                 b.wide, b.flags);
+    }
 }
 
 // Error bits of a finished build, read back on `st`.
@@ -1497,21 +1514,24 @@ aur_status nmh_build_impl(aur_ctx* ctx, const float* V, uint32_t count, aur_nmh*
         }
         delete nmh;
     };
-    // records, permutation and vertices in one allocation (records first: 128-byte aligned)
+    // records, treelet records, permutation and vertices in one allocation (records first: 128-byte aligned)
+    const size_t b_wide = ((size_t)wide_count(nmh->levels) * kWideStride * sizeof(uint4) + 255) & ~(size_t)255;
     const size_t b_recs = ((size_t)n * kRecStride * sizeof(float4) + 255) & ~(size_t)255;
     const size_t b_perm = ((size_t)N * sizeof(uint32_t) + 255) & ~(size_t)255;
-    if (::aur::alloc_device_pool(&nmh->mem, b_recs + b_perm + (size_t)N * 9 * sizeof(float), ctx->nmh_pool->pool, st) !=
-        cudaSuccess) {
+    if (::aur::alloc_device_pool(&nmh->mem, b_recs + b_wide + b_perm + (size_t)N * 9 * sizeof(float),
+                                 ctx->nmh_pool->pool, st) != cudaSuccess) {
         nmh->mem = nullptr;
         cudaGetLastError();
         cleanup();
         return fail(AUR_ERR_OOM, "aur_nmh_build: out of device memory for %u triangles", N);
     }
     nmh->node_recs = (float4*)nmh->mem;
-    nmh->perm = (uint32_t*)((char*)nmh->mem + b_recs);
-    nmh->verts = (float*)((char*)nmh->mem + b_recs + b_perm);
+    nmh->wide = (uint4*)((char*)nmh->mem + b_recs);
+    nmh->perm = (uint32_t*)((char*)nmh->mem + b_recs + b_wide);
+    nmh->verts = (float*)((char*)nmh->mem + b_recs + b_wide + b_perm);
 
     BuildArgs a{V, count, nmh->node_recs, nmh->perm, nmh->verts, nullptr, ctx->d_flags};
+    a.wide = nmh->wide;
     a.lookback_test = ctx->lookback_test;     // armed for this one build only
     ctx->lookback_test = 0;
     if (N <= kGraphMaxTriangles) {
@@ -1548,23 +1568,6 @@ aur_status nmh_build_impl(aur_ctx* ctx, const float* V, uint32_t count, aur_nmh*
         return s;
     }
     nmh->extent = record_extent(root, n);
-    // the records as a linear float4 texture for k_trace (when they fit one);
-    // without it k_trace reads every sector with plain loads
-    int max_linear = 0;
-    if (cudaDeviceGetAttribute(&max_linear, cudaDevAttrMaxTexture1DLinearWidth, ctx->device) == cudaSuccess &&
-        (uint64_t)n * kRecStride <= (uint64_t)max_linear) {
-        cudaResourceDesc rd = {};
-        rd.resType = cudaResourceTypeLinear;
-        rd.res.linear.devPtr = nmh->node_recs;
-        rd.res.linear.desc = cudaCreateChannelDesc<float4>();
-        rd.res.linear.sizeInBytes = (size_t)n * kRecStride * sizeof(float4);
-        cudaTextureDesc td = {};
-        td.readMode = cudaReadModeElementType;
-        if (cudaCreateTextureObject(&nmh->rec_tex, &rd, &td, nullptr) != cudaSuccess) {
-            cudaGetLastError();
-            nmh->rec_tex = 0;
-        }
-    }
     *out = nmh;
     return AUR_OK;
 }

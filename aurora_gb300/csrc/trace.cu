@@ -1,28 +1,23 @@
 // trace.cu — closest-hit and any-hit traversal of the NMH pair-heap.
 //
-// Same visit order and arithmetic as intersect() / intersectAny()
-// (kernels/lib/intersect.cuh:36-152): depth-first, near child first by the
-// sign of the ray direction on the child's axis, range clipped cumulatively
-// by each node's slab (ray.cuh:225-237), Moller-Trumbore with culling
-// (ray.cuh:198-223). The node of the reference is 72 scattered bytes read
-// with 24 scalar loads; here it is a 128-byte record (slab, two triangles as
-// v1, e1, e2, and the subtree boxes of both children) read as one 16-byte
-// load for the slab test, four more only when the slab is hit and three more
-// for the children's boxes before descending. The traversal stack lives in
-// shared memory: the near child is visited next, only the far child is
-// pushed, so the stack never holds more entries than the heap has levels.
-//
-// A trace is two launches. k_trace_packets takes the rays in chunks of 32
-// consecutive rays and traverses each chunk whose rays share a direction
-// octant as one warp packet (one node at a time for the whole warp, each
-// lane with its own decisions: coherent rays share the node fetches); the
-// other chunks go to k_trace, which traverses one ray per lane. Results are
-// the same bit for bit either way.
+// Results of intersect() / intersectAny() (kernels/lib/intersect.cuh:36-152)
+// bit for bit, ties in t to the lower original prim id. A trace runs over the
+// treelet records of aur_wide.cuh in three launches. k_trace_packets takes the
+// rays in chunks of 32 consecutive rays and traverses each chunk whose rays
+// share a direction octant and start close together, as one warp packet when
+// their directions are close too, else one ray per lane; the other chunks go
+// to k_trace_wide, one ray per lane with finished lanes refilled;
+// k_trace_finish checks and stores what both found. A launch that fits the
+// GPU at once does without the second, an NMH of a few triangles without all
+// three (k_trace_tiny). k_trace walks node by node and is what the counting
+// entry points run.
 #include <algorithm>
+#include <cmath>
 
 #include "aur_internal.h"
 #include "aur_math.cuh"
 #include "aur_traverse.cuh"
+#include "aur_wide.cuh"
 
 namespace aur {
 namespace {
@@ -56,27 +51,23 @@ __device__ __forceinline__ void store_result(uint32_t i, uint32_t best, float tm
 
 // First pass of a trace: persistent warps take the rays in chunks of 32
 // consecutive rays (one atomic per warp). A chunk whose rays share their
-// direction octant and start within `packet_span` of each other is
-// traversed as a warp packet (traverse_packet: coherent rays, such as a
-// camera's, share node fetches and lanes); any other chunk goes to the
-// deferred list for k_trace.
+// direction octant and start within `packet_span` of each other stays here:
+// as a warp packet (wide_packet: coherent rays, such as a camera's, share the
+// treelets they meet) when its directions lie within `dir_span`, else one ray
+// per lane (wide_warp). Any other chunk goes to the deferred list for
+// k_trace_wide, or is traversed here too when `small`. Compiled for 6 blocks
+// per SM (80 registers): at 8 the closest-hit form spills (4.9 ms per 8M
+// pinhole rays against 4.3 ms; one node at a time per warp took 7.0 ms).
 template <bool kAny>
-__global__ void __launch_bounds__(kTraceThreads) k_trace_packets(const float4* __restrict__ recs, uint32_t nodes,
-                                                                 const uint32_t* __restrict__ perm,
-                                                                 const float4* __restrict__ rays, uint32_t n,
-                                                                 float4* __restrict__ hits,
+__global__ void __launch_bounds__(kTraceThreads, 6) k_trace_packets(WideView w, const float4* __restrict__ rays,
+                                                                 uint32_t n, float4* __restrict__ hits,
                                                                  uint32_t* __restrict__ occ,
                                                                  uint32_t* __restrict__ ctr,
-                                                                 uint32_t* __restrict__ defer, int cap,
-                                                                 float packet_span) {
-    extern __shared__ uint32_t smem[];
-    const int tid = threadIdx.x;
-    const uint32_t lane = tid & 31;
-    StackRef stk;
-    stk.lo = reinterpret_cast<float*>(smem) + tid;
-    stk.hi = reinterpret_cast<float*>(smem + cap * kTraceThreads) + tid;
-    stk.stride = kTraceThreads;
-    stk.cap = cap;
+                                                                 uint32_t* __restrict__ defer, float packet_span,
+                                                                 float dir_span, bool small) {
+    constexpr WideMode kMode = kAny ? kWideFirst : kWideClosest;
+    __shared__ WideQueue s_queue[kTraceThreads / 32];
+    const uint32_t lane = threadIdx.x & 31;
     const uint32_t chunks = (uint32_t)(((uint64_t)n + 31) >> 5);
     for (;;) {
         uint32_t c = 0;
@@ -96,39 +87,45 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_packets(const float4* _
         }
         const uint32_t oct = dir_octant(dir);
         const uint32_t oct0 = __shfl_sync(0xffffffffu, oct, 0);
-        if (!__all_sync(0xffffffffu, !valid || oct == oct0) || !(warp_origin_span(pos, valid) <= packet_span)) {
-            if (lane == 0) defer[atomicAdd(ctr + 2, 1u)] = c;
-            continue;
+        const bool mixed = !__all_sync(0xffffffffu, !valid || oct == oct0) || !(warp_span(pos, valid) <= packet_span);
+        if (mixed) {
+            uint32_t e = 0;
+            if (lane == 0) e = atomicAdd(ctr + 2, 1u);
+            if (!small) {
+                if (lane == 0) defer[e] = c;
+                continue;
+            }
         }
-        float best_t = tmax, bu = 0.0f, bv = 0.0f;
-        const uint32_t best = traverse_packet<kAny>(recs, nodes, perm, valid, oct0, pos, dir, best_t, bu, bv, stk);
-        if (valid) store_result<kAny>(i, best, tmax, best_t, bu, bv, perm, hits, occ);
+        WideHit h;
+        if (!mixed && warp_span(dir, valid) <= dir_span) {
+            WideRay r;
+            wide_packet<kMode>(w, valid, oct0, pos, dir, tmax, r, h);
+        } else {
+            wide_warp<kMode>(w, s_queue[threadIdx.x >> 5], valid, pos, dir, tmax, h);
+        }
+        if (valid) {
+            if (kAny) occ[i] = h.best;
+            else hits[i] = make_float4(h.t, h.t2, 0.0f, __uint_as_float(h.best));
+        }
     }
 }
 
-// Persistent traversal kernel with dynamic ray fetch: a lane whose ray is
-// done takes the next unprocessed ray at once (one atomic per warp for all
-// lanes asking together), so warps stay full until the ray pool is drained
-// (Aila & Laine, "Understanding the efficiency of ray traversal on GPUs",
-// HPG'09). Every ray is traversed as intersect()/intersectAny(); kBoxes adds
-// the subtree-box pruning (off only to count the reference's own node visits).
-// kCount adds up node fetches, slab crossings (triangle tests) and crossings
-// of nodes with children (box loads) into counters[0..2].
-// kTex: one sector of each node through the texture path (node_triangles).
-// kDefer: the rays are those of the chunks k_trace_packets deferred
-// (defer[0 .. ctr[2]), 32 consecutive rays each), else rays [0, n).
-// ctr[0] is the ray fetch counter. Compiled for 9 blocks of 128 per SM (56
-// registers): the deferred form otherwise takes 62 registers and 8 blocks,
-// which measured slower.
-template <bool kAny, bool kCount, bool kBoxes, bool kTex, bool kDefer>
+// The counting kernel (roofline accounting): every ray one per lane, node by
+// node. Persistent lanes with dynamic ray fetch: a lane whose ray is done
+// takes the next unprocessed ray at once (one atomic per warp for all lanes
+// asking together; Aila & Laine, "Understanding the efficiency of ray
+// traversal on GPUs", HPG'09). Every ray is traversed as intersect() /
+// intersectAny(); kBoxes adds the subtree-box pruning (off to count the
+// reference's own node visits). Adds up node fetches, slab crossings
+// (triangle tests) and crossings of nodes with children (box loads) into
+// counters[0..2]. ctr[0] is the ray fetch counter.
+template <bool kAny, bool kBoxes>
 __global__ void __launch_bounds__(kTraceThreads, 9) k_trace(const float4* __restrict__ recs, uint32_t nodes,
                                                          const uint32_t* __restrict__ perm,
                                                          const float4* __restrict__ rays, uint32_t n,
                                                          float4* __restrict__ hits, uint32_t* __restrict__ occ,
                                                          unsigned long long* __restrict__ counters,
-                                                         uint32_t* __restrict__ ctr, int cap,
-                                                         cudaTextureObject_t tex,
-                                                         const uint32_t* __restrict__ defer) {
+                                                         uint32_t* __restrict__ ctr, int cap) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x;
     StackRef stk;
@@ -137,8 +134,6 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace(const float4* __rest
     stk.stride = kTraceThreads;
     stk.cap = cap;
     uint32_t visits = 0, crossings = 0, inner = 0;
-    // work items: the rays, or 32 per deferred chunk
-    const uint32_t m = kDefer ? (uint32_t)min((unsigned long long)ctr[2] * 32ull, 0xFFFFFFFFull) : n;
     uint32_t i = kNoRay;
     f3 pos = mk3(0.0f), dir = mk3(0.0f), inv = mk3(0.0f);
     float tmax = 0.0f, best_t = 0.0f, bu = 0.0f, bv = 0.0f;
@@ -153,10 +148,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace(const float4* __rest
             if ((tid & 31) == leader) base = atomicAdd(ctr, (uint32_t)__popc(am));
             base = __shfl_sync(am, base, leader);
             i = base + __popc(am & lanemask_lt());
-            if (i >= m) break;
-            // A deferred chunk's positions past the last ray trace the last
-            // ray again (the same result, stored twice).
-            if (kDefer) i = min(defer[i >> 5] * 32u + (i & 31u), n - 1u);
+            if (i >= n) break;
             const float4 r0 = rays[2 * (size_t)i];
             const float4 r1 = rays[2 * (size_t)i + 1];
             pos = mk3(r0.x, r0.y, r0.z);
@@ -172,11 +164,9 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace(const float4* __rest
         float nlo, nhi;
         bool done;
         if (trav_next(s, recs, nodes, pos, dir, inv, best_t, stk, s0, nlo, nhi, visits)) {
-            if (kCount) {
-                ++crossings;
-                inner += 2 * s.k + 1 < nodes;
-            }
-            done = node_triangles<kAny, kTex>(recs, s.k, s0, perm, pos, dir, best_t, bu, bv, best, q5, tex);
+            ++crossings;
+            inner += 2 * s.k + 1 < nodes;
+            done = node_triangles<kAny>(recs, s.k, s0, perm, pos, dir, best_t, bu, bv, best, q5);
             if (!done) trav_descend<kBoxes>(s, recs, q5, pos, dir, inv, best_t, nodes, stk, nlo, nhi);
         } else {
             done = true;
@@ -186,11 +176,210 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace(const float4* __rest
             i = kNoRay;
         }
     }
-    if (kCount) {
-        atomicAdd(counters, (unsigned long long)visits);
-        atomicAdd(counters + 1, (unsigned long long)crossings);
-        atomicAdd(counters + 2, (unsigned long long)inner);
+    atomicAdd(counters, (unsigned long long)visits);
+    atomicAdd(counters + 1, (unsigned long long)crossings);
+    atomicAdd(counters + 2, (unsigned long long)inner);
+}
+
+// The deferred chunks, one ray per lane over the treelets: a lane takes one
+// treelet a step (wide_visit), the warp tests the triangles its lanes met 32
+// at a time (WideQueue). Lanes whose ray is done store the raw result (closest
+// hit: t, t2, NMH position; any hit: NMH position) and are refilled once
+// kRefill of them wait. Compiled for 8 blocks per SM (64 registers, none
+// spilled): what bounds it is latency and the issue slots (the box tests'
+// integer pipe), not memory. Per 8M random rays over 1M triangles, closest
+// hit: 4, 6, 7, 8, 9 and 10 blocks per SM 11.3, 10.5, 10.0, 9.5, 9.7 and 10.0
+// ms; refilled at 1, 2, 4, 6 and 8 waiting lanes 10.1, 9.6, 9.3, 9.4 and 9.5
+// ms; triangles tested by the lane that met them instead of the queue 12.2
+// ms; the node-by-node kernel it replaces 18.3 ms. Any hit, 4M rays toward a
+// light: 7.2 ms before, 3.8 ms now.
+constexpr int kRefill = 4;
+
+template <bool kAny>
+__global__ void __launch_bounds__(kTraceThreads, 8) k_trace_wide(WideView w, const float4* __restrict__ rays, uint32_t n,
+                                                                 float4* __restrict__ hits, uint32_t* __restrict__ occ,
+                                                                 uint32_t* __restrict__ ctr,
+                                                                 const uint32_t* __restrict__ defer) {
+    constexpr WideMode kMode = kAny ? kWideFirst : kWideClosest;
+    __shared__ WideQueue s_queue[kTraceThreads / 32];
+    WideQueue& q = s_queue[threadIdx.x >> 5];
+    const uint32_t m = (uint32_t)min((unsigned long long)ctr[2] * 32ull, 0xFFFFFFFFull);
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t i = kNoRay, count = 0, seq = 0;
+    bool running = false, pool = true;
+    WideRay r;
+    WideState s;
+    float lim = 0.0f;
+    wide_ray(r, mk3(0.0f), mk3(0.0f));
+    wide_init(s, w.levels);
+    for (;;) {
+        const uint32_t run = __ballot_sync(0xffffffffu, running);
+        if (run == 0u || (pool && __popc(run) <= 32 - kRefill)) {
+            queue_test<kMode>(q, lane, count, count, w);
+            count = 0;
+            if (!running && i != kNoRay) {
+                if (kAny) occ[i] = q.best[lane];
+                else hits[i] = make_float4(__uint_as_float((uint32_t)(q.key[lane] >> 32)), __uint_as_float(q.t2[lane]),
+                                           0.0f, __uint_as_float(q.best[lane]));
+                i = kNoRay;
+            }
+            if (pool) {
+                const uint32_t want = ~run;
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(ctr, (uint32_t)__popc(want));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                pool = base < m && m - base > (uint32_t)__popc(want);
+                const uint32_t j = base + __popc(want & lanemask_lt());
+                if (!running && j >= base && j < m) {
+                    // a chunk's positions past the last ray trace the last ray again (the same result, stored twice)
+                    i = min(defer[j >> 5] * 32u + (j & 31u), n - 1u);
+                    const float4 r0 = rays[2 * (size_t)i];
+                    const float4 r1 = rays[2 * (size_t)i + 1];
+                    WideHit h;
+                    running = wide_begin(r, s, h, w, mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), r0.w);
+                    queue_ray<kMode>(q, lane, r.pos, r.dir, r0.w);
+                    lim = r0.w;
+                    seq = 0;
+                }
+            }
+            if (!__any_sync(0xffffffffu, running || i != kNoRay)) break;
+        }
+        uint32_t tris = 0;
+        if (running) tris = wide_visit<kMode>(w, r, s, lim);
+        queue_add<kMode>(q, lane, count, seq, tris, r, s, w);
+        if (running) {
+            if (kAny) running = q.key[lane] == kNoKey && wide_next<kMode>(r, s);
+            else {
+                lim = __uint_as_float((uint32_t)(q.key[lane] >> 32));
+                running = wide_next<kMode>(r, s);
+            }
+        }
     }
+}
+
+// Turns what the traversals left in the result buffers (closest hit: t, t2,
+// NMH position; any hit: NMH position) into results, checked against the walk
+// of intersect() (finish_closest, finish_any) and stored as store_result
+// does. Kept apart from the traversals: there the checks would run for a few
+// lanes at a time and cost the loop registers (a spill in every step and up
+// to twice k_trace_wide's time).
+template <bool kAny>
+__global__ void __launch_bounds__(kTraceThreads) k_trace_finish(WideView w, const float4* __restrict__ rays, uint32_t n,
+                                                                float4* __restrict__ hits,
+                                                                uint32_t* __restrict__ occ) {
+    const uint32_t step = gridDim.x * kTraceThreads;
+    for (uint64_t k = blockIdx.x * kTraceThreads + threadIdx.x; k < n; k += step) {
+        const uint32_t i = (uint32_t)k;
+        const float4 r0 = rays[2 * (size_t)i];
+        const float4 r1 = rays[2 * (size_t)i + 1];
+        WideRay r;
+        r.pos = mk3(r0.x, r0.y, r0.z);
+        r.dir = mk3(r1.x, r1.y, r1.z);
+        WideHit h;
+        h.t = h.t2 = 0.0f;
+        float u = 0.0f, v = 0.0f;
+        if (kAny) {
+            h.best = finish_any(w, r, occ[i], r0.w);
+        } else {
+            const float4 raw = hits[i];
+            h.t = raw.x;
+            h.t2 = raw.y;
+            h.best = __float_as_uint(raw.w);
+            finish_closest(w, r, h, r0.w, u, v);
+        }
+        store_result<kAny>(i, h.best, r0.w, h.t, u, v, w.perm, hits, occ);
+    }
+}
+
+// An NMH of at most kTinyTris triangles has no use for a tree: every lane
+// tests every triangle, staged in shared memory and read by the whole warp at
+// one address, so no lane waits for another's path and no load waits for a
+// node. Any hit collects the accepted triangles and takes the one whose node
+// intersectAny() visits first for the ray's octant (preorder ranks, near child
+// first). One launch; the results are checked as k_trace_finish does.
+constexpr uint32_t kTinyTris = 64;
+
+template <bool kAny>
+__global__ void __launch_bounds__(kTraceThreads) k_trace_tiny(WideView w, uint32_t count,
+                                                              const float4* __restrict__ rays, uint32_t n,
+                                                              float4* __restrict__ hits, uint32_t* __restrict__ occ,
+                                                              uint32_t* __restrict__ ctr) {
+    __shared__ float4 s_tri[kTinyTris][3];                 // v1, e1, e2; the first's w: prim id
+    __shared__ uint8_t s_rank[8][kTinyTris / 2];
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[2] = 0u;  // no chunk is deferred
+    for (uint32_t j = threadIdx.x; j < count; j += blockDim.x) {
+        const float* q = w.verts + (size_t)j * 9;
+        s_tri[j][0] = make_float4(q[0], q[3], q[6], __uint_as_float(w.perm[j]));
+        s_tri[j][1] = make_float4(q[1] - q[0], q[4] - q[3], q[7] - q[6], 0.0f);
+        s_tri[j][2] = make_float4(q[2] - q[0], q[5] - q[3], q[8] - q[6], 0.0f);
+    }
+    if (kAny) {
+        for (uint32_t j = threadIdx.x; j < 8u * w.nodes; j += blockDim.x) {
+            const uint32_t oct = j & 7u, node = j >> 3, lvl = 31u - (uint32_t)__clz(node + 1u);
+            uint32_t rank = 0;
+            for (uint32_t l = 1; l <= lvl; ++l) {          // down the path: the node before, and a far child's sibling
+                const uint32_t k = ((node + 1u) >> (lvl - l)) - 1u;
+                const bool second = !(k & 1u), far = second != (((oct >> (l % 3u)) & 1u) != 0u);
+                uint32_t size = 0;                         // of the sibling's subtree
+                if (far)
+                    for (uint32_t f = second ? k - 1u : k + 1u, m = 1; f < w.nodes; f = 2u * f + 1u, m <<= 1)
+                        size += min(m, w.nodes - f);
+                rank += 1u + size;
+            }
+            s_rank[oct][node] = (uint8_t)rank;
+        }
+    }
+    __syncthreads();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 r0 = rays[2 * (size_t)i];
+    const float4 r1 = rays[2 * (size_t)i + 1];
+    WideRay r;
+    r.pos = mk3(r0.x, r0.y, r0.z);
+    r.dir = mk3(r1.x, r1.y, r1.z);
+    WideHit h;
+    h.t = h.t2 = r0.w;
+    h.best = kNoPrim;
+    uint32_t best_id = 0u;
+    uint64_t met = 0;
+    for (uint32_t j = 0; j < count; ++j) {
+        const float4 a = s_tri[j][0], b = s_tri[j][1], c = s_tri[j][2];
+        float u, v, t;
+        if (!intersect_tri(r.pos, r.dir, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), mk3(c.x, c.y, c.z), u, v, t)) continue;
+        if (!(t > kEpsilon)) continue;
+        const uint32_t id = __float_as_uint(a.w);
+        if (kAny) {
+            if (t < h.t) met |= 1ull << j;
+        } else if (t < h.t) {
+            h.t2 = h.t;
+            h.t = t;
+            h.best = j;
+            best_id = id;
+        } else {
+            if (t == h.t && h.best != kNoPrim && id < best_id) {
+                h.best = j;
+                best_id = id;
+            }
+            h.t2 = fminf(h.t2, t);
+        }
+    }
+    if (kAny) {
+        const uint32_t oct = dir_octant(r.dir);
+        uint32_t first = ~0u;
+        while (met) {
+            const uint32_t j = (uint32_t)__ffsll((long long)met) - 1u;
+            met &= met - 1ull;
+            first = min(first, ((uint32_t)s_rank[oct][j >> 1] << 8) | j);
+        }
+        if (first != ~0u) h.best = first & 255u;
+        occ[i] = h.best;
+    } else {
+        hits[i] = make_float4(h.t, h.t2, 0.0f, __uint_as_float(h.best));
+    }
+    float u = 0.0f, v = 0.0f;
+    if (kAny) h.best = finish_any(w, r, h.best, r0.w);
+    else finish_closest(w, r, h, r0.w, u, v);
+    store_result<kAny>(i, h.best, r0.w, h.t, u, v, w.perm, hits, occ);
 }
 
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
@@ -202,6 +391,20 @@ inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b
 // and one ray per lane is faster for them.
 inline float packet_span(const aur_nmh* nmh) { return nmh->extent * (1.0f / 64.0f); }
 
+// Largest spread of a packet's directions (per component): about two and a
+// half times the angle that one of the soup's count^(1/3) cells along a side
+// takes at the distance of its extent. Wider packets meet many more treelets
+// than each of their rays does. 1M triangles (0.025): a 2.8k-pixel-wide pinhole's
+// rows (spread 0.011) 4.3 ms as packets against 7.0 ms one ray per lane, a
+// 1k-wide one's (0.032) 1.32 against 1.36, a 512-wide one's (0.06) 0.91 against
+// 0.62, a 200-wide one's (0.16) 1.1 against 0.21. 30k triangles (0.08): 0.60
+// against 0.83 (0.032) and 0.40 against 0.45 (0.06).
+inline float dir_span(const aur_nmh* nmh) { return 2.5f / cbrtf((float)std::max(nmh->count, 1u)); }
+
+// Up to this many rays per SM are in flight at once in k_trace_packets, so
+// nothing is gained by handing the mixed chunks to a second launch.
+constexpr uint32_t kSmallPerSm = 6 * kTraceThreads;
+
 template <typename K>
 aur_status persistent_grid(aur_ctx* ctx, K kernel, size_t smem, uint32_t n, uint32_t& grid) {
     int per_sm = 0;
@@ -210,25 +413,37 @@ aur_status persistent_grid(aur_ctx* ctx, K kernel, size_t smem, uint32_t n, uint
     return AUR_OK;
 }
 
-// The counting kernels (roofline accounting) trace every ray per lane and
-// never read through the texture path; the shipped trace is two launches:
-// k_trace_packets over all rays, then k_trace over the chunks it deferred.
-template <bool kAny, bool kCount, bool kBoxes, bool kTex>
-aur_status launch_kernel(aur_ctx* ctx, const aur_nmh* nmh, const float4* r, uint32_t n, float4* h, uint32_t* occ,
-                         unsigned long long* counters, cudaStream_t stream, int slot) {
+// The counting kernel over every ray.
+template <bool kAny, bool kBoxes>
+aur_status launch_count(aur_ctx* ctx, const aur_nmh* nmh, const float4* r, uint32_t n, float4* h, uint32_t* occ,
+                        unsigned long long* counters, cudaStream_t stream, int slot) {
     const int cap = (int)nmh->levels + 1;
     const size_t smem = (size_t)2 * cap * kTraceThreads * sizeof(uint32_t);
     uint32_t* ctr = ctx->d_flags + 16 + 4 * slot;
     AUR_CUDA(cudaMemsetAsync(ctr, 0, 3 * sizeof(uint32_t), stream));
     uint32_t grid = 0;
-    if constexpr (kCount) {
-        aur_status st = persistent_grid(ctx, k_trace<kAny, kCount, kBoxes, kTex, false>, smem, n, grid);
-        if (st != AUR_OK) return st;
-        k_trace<kAny, kCount, kBoxes, kTex, false><<<grid, kTraceThreads, smem, stream>>>(
-            nmh->node_recs, nmh->nodes, nmh->perm, r, n, h, occ, counters, ctr, cap, nmh->rec_tex, nullptr);
+    const aur_status st = persistent_grid(ctx, k_trace<kAny, kBoxes>, smem, n, grid);
+    if (st != AUR_OK) return st;
+    k_trace<kAny, kBoxes><<<grid, kTraceThreads, smem, stream>>>(nmh->node_recs, nmh->nodes, nmh->perm, r, n, h, occ,
+                                                                 counters, ctr, cap);
+    AUR_CUDA(cudaGetLastError());
+    return AUR_OK;
+}
+
+// The shipped trace: k_trace_packets over all rays, then k_trace_wide and
+// k_trace_finish over the chunks it deferred.
+template <bool kAny>
+aur_status launch_wide(aur_ctx* ctx, const aur_nmh* nmh, const float4* r, uint32_t n, float4* h, uint32_t* occ,
+                       cudaStream_t stream, int slot) {
+    uint32_t* ctr = ctx->d_flags + 16 + 4 * slot;
+    const WideView w = wide_view(nmh);
+    if (nmh->count <= kTinyTris) {
+        const uint32_t threads = n <= (uint32_t)ctx->sm_count * 64u ? 32u : kTraceThreads;   // a block per SM when they are few
+        k_trace_tiny<kAny><<<cdiv(n, threads), threads, 0, stream>>>(w, nmh->count, r, n, h, occ, ctr);
         AUR_CUDA(cudaGetLastError());
         return AUR_OK;
     }
+    AUR_CUDA(cudaMemsetAsync(ctr, 0, 3 * sizeof(uint32_t), stream));
     Scratch& d = ctx->defer[slot];
     const size_t need = (size_t)cdiv(n, 32) * sizeof(uint32_t);
     if (d.bytes < need) {
@@ -240,27 +455,23 @@ aur_status launch_kernel(aur_ctx* ctx, const aur_nmh* nmh, const float4* r, uint
         d.bytes = need;
     }
     uint32_t* defer = static_cast<uint32_t*>(d.ptr);
-    aur_status st = persistent_grid(ctx, k_trace_packets<kAny>, smem, n, grid);
+    uint32_t grid = 0;
+    aur_status st = persistent_grid(ctx, k_trace_packets<kAny>, 0, n, grid);
     if (st != AUR_OK) return st;
-    k_trace_packets<kAny><<<grid, kTraceThreads, smem, stream>>>(nmh->node_recs, nmh->nodes, nmh->perm, r, n, h, occ,
-                                                                  ctr, defer, cap, packet_span(nmh));
+    const bool small = n <= (uint32_t)ctx->sm_count * kSmallPerSm;
+    k_trace_packets<kAny><<<grid, kTraceThreads, 0, stream>>>(w, r, n, h, occ, ctr, defer, packet_span(nmh), dir_span(nmh), small);
     AUR_CUDA(cudaGetLastError());
-    st = persistent_grid(ctx, k_trace<kAny, false, kBoxes, kTex, true>, smem, n, grid);
+    if (!small) {
+        st = persistent_grid(ctx, k_trace_wide<kAny>, 0, n, grid);
+        if (st != AUR_OK) return st;
+        k_trace_wide<kAny><<<grid, kTraceThreads, 0, stream>>>(w, r, n, h, occ, ctr, defer);
+        AUR_CUDA(cudaGetLastError());
+    }
+    st = persistent_grid(ctx, k_trace_finish<kAny>, 0, n, grid);
     if (st != AUR_OK) return st;
-    k_trace<kAny, false, kBoxes, kTex, true><<<grid, kTraceThreads, smem, stream>>>(
-        nmh->node_recs, nmh->nodes, nmh->perm, r, n, h, occ, nullptr, ctr, cap, nmh->rec_tex, defer);
+    k_trace_finish<kAny><<<grid, kTraceThreads, 0, stream>>>(w, r, n, h, occ);
     AUR_CUDA(cudaGetLastError());
     return AUR_OK;
-}
-
-// The shipped kernels read through the texture path when the NMH has its
-// record texture; the counting kernels (roofline accounting) never do.
-template <bool kAny, bool kCount, bool kBoxes = true>
-aur_status launch_one(aur_ctx* ctx, const aur_nmh* nmh, const float4* r, uint32_t n, float4* h, uint32_t* occ,
-                      unsigned long long* counters, cudaStream_t stream, int slot) {
-    if (!kCount && nmh->rec_tex)
-        return launch_kernel<kAny, kCount, kBoxes, true>(ctx, nmh, r, n, h, occ, counters, stream, slot);
-    return launch_kernel<kAny, kCount, kBoxes, false>(ctx, nmh, r, n, h, occ, counters, stream, slot);
 }
 
 aur_status launch_trace(aur_ctx* ctx, const aur_nmh* nmh, const aur_ray* rays, uint32_t n, aur_hit* hits,
@@ -270,13 +481,13 @@ aur_status launch_trace(aur_ctx* ctx, const aur_nmh* nmh, const aur_ray* rays, u
     const float4* r = reinterpret_cast<const float4*>(rays);
     float4* h = reinterpret_cast<float4*>(hits);
     if (counters && !pruned)
-        return occluder ? launch_one<true, true, false>(ctx, nmh, r, n, nullptr, occluder, counters, stream, slot)
-                        : launch_one<false, true, false>(ctx, nmh, r, n, h, nullptr, counters, stream, slot);
+        return occluder ? launch_count<true, false>(ctx, nmh, r, n, nullptr, occluder, counters, stream, slot)
+                        : launch_count<false, false>(ctx, nmh, r, n, h, nullptr, counters, stream, slot);
     if (counters)
-        return occluder ? launch_one<true, true>(ctx, nmh, r, n, nullptr, occluder, counters, stream, slot)
-                        : launch_one<false, true>(ctx, nmh, r, n, h, nullptr, counters, stream, slot);
-    return occluder ? launch_one<true, false>(ctx, nmh, r, n, nullptr, occluder, nullptr, stream, slot)
-                    : launch_one<false, false>(ctx, nmh, r, n, h, nullptr, nullptr, stream, slot);
+        return occluder ? launch_count<true, true>(ctx, nmh, r, n, nullptr, occluder, counters, stream, slot)
+                        : launch_count<false, true>(ctx, nmh, r, n, h, nullptr, counters, stream, slot);
+    return occluder ? launch_wide<true>(ctx, nmh, r, n, nullptr, occluder, stream, slot)
+                    : launch_wide<false>(ctx, nmh, r, n, h, nullptr, stream, slot);
 }
 
 }  // namespace aur

@@ -289,7 +289,7 @@ __device__ __forceinline__ bool packet_or_defer(const WfArgs& a, uint32_t* defer
     scene0 = __shfl_sync(0xffffffffu, scene, 0);
     oct0 = __shfl_sync(0xffffffffu, oct, 0);
     if (__all_sync(0xffffffffu, !valid || (scene == scene0 && oct == oct0)) &&
-        warp_origin_span(pos, valid) <= a.scenes[scene0].packet_span)
+        warp_span(pos, valid) <= a.scenes[scene0].packet_span)
         return true;
     if (lane_id() == 0) a.defer[atomicAdd(defer_count, 1u)] = chunk;
     return false;

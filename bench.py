@@ -10,15 +10,16 @@ the metric is Mrays/s closest-hit. Inputs are seeded synthetic data.
 
 Prints one JSON line. `e2e` measures the same metric through the C ABI's
 host-buffer call (aur_trace_closest_host: rays copied in from pinned host
-memory and hits copied back inside the timed region). A trace is two
+memory and hits copied back inside the timed region). A trace is three
 launches: warp packets for the 32-ray chunks of one direction octant (the
-pinhole half), then one ray per thread for the other chunks. `roofline`
+pinhole half), treelets one ray per lane for the other chunks, and the pass
+that checks those. `roofline`
 divides the algorithmic bytes of a trace by its CUDA-event duration, with the
 reference algorithm's bytes: 24 B ray in + 16 B hit out + 72 B per node that
 the reference's intersect() visits (two triangles of 36 B), the visits
 counted by the same traversal without box pruning. This traversal's own
 reads per ray (fewer nodes, 128-byte records) are reported beside it, and
-the DRAM traffic of one trace (both launches) from the committed ncu summary
+the DRAM traffic of one trace (all launches) from the committed ncu summary
 when that summary was captured from the current traversal sources. `cpu_baseline` times the
 oracle's C++ restatement of the reference traversal on a sample of the same
 rays on all host cores. With --gpus N > 1 (under torchrun) every rank runs
@@ -299,7 +300,7 @@ def load_traffic():
                       % (TRAFFIC_PROFILE, vals.get("source_sha256_16", "(unrecorded)"), now))
     try:
         return int(vals["traffic_bytes_per_trace"]), "%s (ncu dram__bytes_read.sum + dram__bytes_write.sum of " \
-            "both launches of a trace, traversal sources %s)" % (TRAFFIC_PROFILE, now)
+            "all launches of a trace, traversal sources %s)" % (TRAFFIC_PROFILE, now)
     except (KeyError, ValueError):
         return None, "no traffic_bytes_per_trace line in %s" % TRAFFIC_PROFILE
 
@@ -1015,9 +1016,9 @@ def main():
                      "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)",
                      "definition": "reference algorithm bytes per trace: 24 B ray in + 16 B hit out + 72 B per node "
                                    "the reference's intersect() visits (counted by this traversal without box "
-                                   "pruning), divided by the average CUDA-event time of a trace call (its two "
-                                   "launches: the warp-packet pass and the one-ray-per-thread pass over the "
-                                   "chunks it deferred)",
+                                   "pruning), divided by the average CUDA-event time of a trace call (its three "
+                                   "launches: the warp-packet pass, the treelet pass over the chunks it "
+                                   "deferred and the pass that checks those)",
                      "algorithmic_bytes_per_launch": ref_bytes,
                      "reference_node_visits_per_ray": visits_closest / N_RAYS,
                      "dram_GBps": traffic / avg_launch_s / 1e9 if traffic else None,
@@ -1031,7 +1032,7 @@ def main():
                      "slab_crossings_per_ray": wc["slab_crossings"] / N_RAYS},
         "e2e": {"value": e2e_value, "unit": "Mrays/s", "h2d_bytes_per_step": N_RAYS * 32,
                 "d2h_bytes_per_step": N_RAYS * 16, "matches_device_result": bool(same)},
-        "gpu_launches": 2 * args.steps,    # k_trace_packets + k_trace per step
+        "gpu_launches": 3 * args.steps,    # k_trace_packets, k_trace_wide, k_trace_finish per step
         "clocks": clocks,
         "any_hit": {"value": world * N_RAYS / (any_ms * 1e-3) / 1e6, "unit": "Mrays/s", "ms_per_step": any_ms,
                     "node_fetches_per_ray": work["any"]["node_fetches"] / N_RAYS,

@@ -242,15 +242,12 @@ aur_status aur_nmh_build(aur_ctx* ctx, const float* vertices, uint32_t count, au
  * purpose: that build returns AUR_ERR_TIMEOUT and creates no NMH. Soups of
  * at most 4,096 triangles have no such wait and build normally. */
 aur_status aur_debug_lookback_timeout(aur_ctx* ctx, uint32_t spins);
-/* Test hook (no counterpart in the reference): the NMH's node records are
- * bound as a texture at build, and the traversal entry points read part of
- * each node through it; an NMH too large for a texture (over about 33M
- * triangles) is traversed with plain loads only. This drops the texture of
- * `nmh` (after synchronizing its device), so that tests can compare both
- * paths on small soups. */
+/* Test hook kept for its callers: the traversal once read part of each node
+ * through a texture, which this dropped. It no longer has one; checks `nmh`
+ * and does nothing. */
 aur_status aur_debug_nmh_drop_texture(aur_nmh* nmh);
-/* Frees the NMH (its records, permutation and vertices, and the records'
- * texture). Synchronizes the NMH's device first: no launch may still be
+/* Frees the NMH (its records, permutation and vertices).
+ * Synchronizes the NMH's device first: no launch may still be
  * reading it. */
 aur_status aur_nmh_destroy(aur_nmh* nmh);
 /* Triangle count after padding and number of heap levels (log2i(count/2)+1). */
@@ -327,7 +324,7 @@ aur_status aur_generate_tb(aur_ctx* ctx, const float* normals, uint32_t count, f
  * taken in chunks of 32 consecutive rays: a chunk whose directions share
  * their octant (signs of x, y, z) is traversed by one warp together, which
  * is fastest for coherent rays (a camera's, rays toward one light); the
- * other chunks are traversed one ray per thread. Results are the same. The
+ * other chunks are traversed one ray per lane over two-level nodes. Results are the same. The
  * first call with more rays than before allocates 4 bytes per 32 rays. */
 aur_status aur_trace_closest(aur_ctx* ctx, const aur_nmh* nmh, const aur_ray* rays, uint32_t n, aur_hit* hits);
 /* Any hit (shadow ray, intersectAny(), intersect.cuh:36-86): occluder[i] is
