@@ -60,11 +60,30 @@ struct WideView {
     const float* verts;       // NMH order, 9 floats per triangle
     uint32_t nodes;           // NMH nodes
     uint32_t levels;          // NMH levels
+
+    // the tree that a lane's ray runs in (WideQueue): the same for all
+    __device__ __forceinline__ const float4* recs_of(uint32_t) const { return recs; }
+    __device__ __forceinline__ const uint32_t* perm_of(uint32_t) const { return perm; }
 };
 
 inline WideView wide_view(const aur_nmh* nmh) {
     return WideView{nmh->node_recs, nmh->wide, nmh->perm, nmh->verts, nmh->nodes, nmh->levels};
 }
+
+// Largest origin spread of a warp packet: 1/64 of the soup's extent. Rays
+// that start further apart visit mostly different nodes near their origins,
+// and one ray per lane is faster for them.
+inline float packet_span(const aur_nmh* nmh) { return nmh->extent * (1.0f / 64.0f); }
+
+// Largest spread of a packet's directions (per component): about two and a
+// half times the angle that one of the soup's count^(1/3) cells along a side
+// takes at the distance of its extent. Wider packets meet many more treelets
+// than each of their rays does. 1M triangles (0.025): a 2.8k-pixel-wide pinhole's
+// rows (spread 0.011) 4.3 ms as packets against 7.0 ms one ray per lane, a
+// 1k-wide one's (0.032) 1.32 against 1.36, a 512-wide one's (0.06) 0.91 against
+// 0.62, a 200-wide one's (0.16) 1.1 against 0.21. 30k triangles (0.08): 0.60
+// against 0.83 (0.032) and 0.40 against 0.45 (0.06).
+inline float dir_span(const aur_nmh* nmh) { return 2.5f / cbrtf((float)(nmh->count ? nmh->count : 1u)); }
 
 // Index of the first treelet with this lvlbit among all records.
 __host__ __device__ __forceinline__ uint32_t wide_base(uint32_t lvlbit, uint32_t levels) {
@@ -473,9 +492,10 @@ __device__ __forceinline__ void queue_ray(WideQueue& q, uint32_t lane, const f3&
     q.t2[lane] = __float_as_uint(tmax);
 }
 
-// Tests the last m (<= 32) waiting pairs. Call with all lanes.
-template <WideMode kMode>
-__device__ __forceinline__ void queue_test(WideQueue& q, uint32_t lane, uint32_t count, uint32_t m, const WideView& w) {
+// Tests the last m (<= 32) waiting pairs; `w` tells each lane's tree (WideView,
+// or one tree per lane). Call with all lanes.
+template <WideMode kMode, typename Trees>
+__device__ __forceinline__ void queue_test(WideQueue& q, uint32_t lane, uint32_t count, uint32_t m, const Trees& w) {
     __syncwarp();
     uint32_t own = 0, idx = 0;
     unsigned long long mine = kNoKey;
@@ -486,10 +506,10 @@ __device__ __forceinline__ void queue_test(WideQueue& q, uint32_t lane, uint32_t
         const float4 a = q.pd[own];
         const float2 b = q.d[own];
         float t;
-        if (wide_tri(w.recs, idx, mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y), t)) {
+        if (wide_tri(w.recs_of(own), idx, mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y), t)) {
             if (kMode == kWideClosest) {
                 if (t <= __uint_as_float(q.t2[own])) {
-                    const unsigned long long k = ((unsigned long long)__float_as_uint(t) << 32) | w.perm[idx];
+                    const unsigned long long k = ((unsigned long long)__float_as_uint(t) << 32) | w.perm_of(own)[idx];
                     const unsigned long long old = atomicMin(&q.key[own], k);
                     if (k < old) mine = k;
                     atomicMin(&q.t2[own], (uint32_t)((k < old ? old : k) >> 32));
@@ -507,9 +527,9 @@ __device__ __forceinline__ void queue_test(WideQueue& q, uint32_t lane, uint32_t
 
 // Adds the triangles of each lane's `tris` (wide_visit) to the queue, testing
 // 32 pairs whenever that many wait. count and seq as left by the last call.
-template <WideMode kMode>
+template <WideMode kMode, typename Trees>
 __device__ __forceinline__ void queue_add(WideQueue& q, uint32_t lane, uint32_t& count, uint32_t& seq, uint32_t tris,
-                                          const WideRay& r, const WideState& s, const WideView& w) {
+                                          const WideRay& r, const WideState& s, const Trees& w) {
     for (;;) {
         const uint32_t have = __ballot_sync(0xffffffffu, tris != 0u);
         if (have == 0u) break;

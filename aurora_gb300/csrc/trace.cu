@@ -12,7 +12,6 @@
 // three (k_trace_tiny). k_trace walks node by node and is what the counting
 // entry points run.
 #include <algorithm>
-#include <cmath>
 
 #include "aur_internal.h"
 #include "aur_math.cuh"
@@ -385,21 +384,6 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_tiny(WideView w, uint32
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 }  // namespace
-
-// Largest origin spread of a warp packet: 1/64 of the soup's extent. Rays
-// that start further apart visit mostly different nodes near their origins,
-// and one ray per lane is faster for them.
-inline float packet_span(const aur_nmh* nmh) { return nmh->extent * (1.0f / 64.0f); }
-
-// Largest spread of a packet's directions (per component): about two and a
-// half times the angle that one of the soup's count^(1/3) cells along a side
-// takes at the distance of its extent. Wider packets meet many more treelets
-// than each of their rays does. 1M triangles (0.025): a 2.8k-pixel-wide pinhole's
-// rows (spread 0.011) 4.3 ms as packets against 7.0 ms one ray per lane, a
-// 1k-wide one's (0.032) 1.32 against 1.36, a 512-wide one's (0.06) 0.91 against
-// 0.62, a 200-wide one's (0.16) 1.1 against 0.21. 30k triangles (0.08): 0.60
-// against 0.83 (0.032) and 0.40 against 0.45 (0.06).
-inline float dir_span(const aur_nmh* nmh) { return 2.5f / cbrtf((float)std::max(nmh->count, 1u)); }
 
 // Up to this many rays per SM are in flight at once in k_trace_packets, so
 // nothing is gained by handing the mixed chunks to a second launch.

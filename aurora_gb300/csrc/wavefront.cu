@@ -32,6 +32,7 @@
 
 #include "aur_integrate.cuh"
 #include "aur_internal.h"
+#include "aur_wide.cuh"
 
 namespace aur {
 namespace {
@@ -49,7 +50,7 @@ constexpr uint32_t kWfErrStack = 4u;
 constexpr uint32_t kWfStack = AUR_MAX_DEPTH + 2;
 // Largest block of the stage kernels: the traversal and shading stages are
 // compiled for it with at most 64 registers (4 blocks of 256 per SM), which
-// measured faster than their unconstrained 70-72 registers.
+// measured faster than more, the packet stage for 80.
 constexpr int kWfMaxBlock = 256;
 
 struct WfScene {
@@ -69,7 +70,9 @@ struct WfScene {
     const float* mis_pa;
     uint32_t mis_count;
     uint32_t nodes;
-    float packet_span;   // largest origin spread of a warp packet (1/64 of the soup's extent)
+    uint32_t levels;
+    const uint4* wide;   // treelet records
+    float packet_span, dir_span;   // largest origin and direction spread of a warp packet
     uint32_t num_lights;
     uint32_t width, height;
     uint32_t pix_off;
@@ -104,13 +107,12 @@ struct WfArgs {
     uint32_t Q;                   // paths in flight
     uint32_t M;                   // light-sample slots per path
     uint32_t spp, max_depth, mode, seed;
-    int cap;                      // traversal stack entries
     // path state, indexed by pool slot
     float4* o;      // origin
     float4* d;      // direction
     float4* thr;    // throughput, w = density of the bounce that made the ray (0: camera ray)
     float4* col;    // colour, w = any hit
-    float4* hit;    // t, u, v, tri
+    float4* hit;    // t, u, v, tri (between extend and its finish: t, t2, -, tri)
     uint4* meta;    // item, depth, ray index, scene
     float4* ndir;   // bounce direction, w = 1 if the path continues
     float4* nthr;   // bounce throughput, w = the bounce's density (AUR_MODE_PATH_MIS)
@@ -147,14 +149,23 @@ __device__ __forceinline__ uint32_t agg_inc(uint32_t* ctr) {
     return base + __popc(m & lt);
 }
 
-__device__ __forceinline__ StackRef wf_stack(uint32_t* smem, int cap) {
-    StackRef s;
-    s.lo = reinterpret_cast<float*>(smem) + threadIdx.x;
-    s.hi = reinterpret_cast<float*>(smem + cap * blockDim.x) + threadIdx.x;
-    s.stride = blockDim.x;
-    s.cap = cap;
-    return s;
+__device__ __forceinline__ WideView scene_tree(const WfScene& sc) {
+    return WideView{sc.recs, sc.wide, sc.perm, sc.verts, sc.nodes, sc.levels};
 }
+
+// The trees of a warp whose lanes' rays run in different scenes.
+struct WfTrees {
+    const WfScene* scenes;
+    const uint32_t* scene;   // per lane, in shared memory
+    __device__ __forceinline__ const float4* recs_of(uint32_t lane) const { return scenes[scene[lane]].recs; }
+    __device__ __forceinline__ const uint32_t* perm_of(uint32_t lane) const { return scenes[scene[lane]].perm; }
+};
+
+// Dynamic shared memory of the traversal stages, per warp.
+struct WfWarp {
+    WideQueue q;
+    uint32_t scene[32];
+};
 
 __device__ __forceinline__ uint32_t find_scene(const uint32_t* pix_off, uint32_t n, uint32_t gp) {
     uint32_t lo = 0, hi = n;   // pix_off[lo] <= gp < pix_off[hi]
@@ -267,8 +278,16 @@ __global__ void k_wf_generate_commit(WfArgs a) {
     c->ext_defer = 0;
 }
 
-// Next queue position for a lane that needs work (one atomic per warp).
-__device__ __forceinline__ uint32_t fetch_next(uint32_t* cursor) { return agg_inc(cursor); }
+// Next positions of [0, m) for the lanes of `want` (one atomic per warp; call
+// with all 32 lanes). `pool` becomes false when none are left after these.
+__device__ __forceinline__ uint32_t refill(uint32_t* cursor, uint32_t want, uint32_t m, bool& pool) {
+    uint32_t lt, base = 0;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    if (lane_id() == 0) base = atomicAdd(cursor, (uint32_t)__popc(want));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    pool = base < m && m - base > (uint32_t)__popc(want);
+    return base + __popc(want & lt);
+}
 
 // Takes the next chunk of 32 queue entries for the whole warp (one atomic);
 // returns false when the n entries are exhausted.
@@ -289,19 +308,17 @@ __device__ __forceinline__ bool packet_or_defer(const WfArgs& a, uint32_t* defer
     scene0 = __shfl_sync(0xffffffffu, scene, 0);
     oct0 = __shfl_sync(0xffffffffu, oct, 0);
     if (__all_sync(0xffffffffu, !valid || (scene == scene0 && oct == oct0)) &&
-        warp_span(pos, valid) <= a.scenes[scene0].packet_span)
+        warp_span(pos, valid) <= a.scenes[scene0].packet_span && warp_span(dir, valid) <= a.scenes[scene0].dir_span)
         return true;
     if (lane_id() == 0) a.defer[atomicAdd(defer_count, 1u)] = chunk;
     return false;
 }
 
 // Closest hit, first pass: chunks of 32 queued paths of one scene and one
-// direction octant (the camera rays of an 8x4 pixel tile, say) are
-// traversed as warp packets (traverse_packet); the other chunks are left to
-// k_wf_extend. Same results either way.
-__global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_extend_packets(WfArgs a) {
-    extern __shared__ uint32_t smem[];
-    const StackRef stk = wf_stack(smem, a.cap);
+// direction octant with close origins and directions (the camera rays of an
+// 8x4 pixel tile, say) are traversed as warp packets (wide_packet); the other
+// chunks are left to k_wf_extend. Same results either way.
+__global__ void __launch_bounds__(kWfMaxBlock, 3) k_wf_extend_packets(WfArgs a) {
     WfCtl* c = a.ctl;
     const uint32_t cur = c->iter & 1u;
     const uint32_t n = c->ext_count[cur];
@@ -320,59 +337,101 @@ __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_extend_packets(WfArgs a) 
         }
         uint32_t scene0, oct0;
         if (!packet_or_defer(a, &c->ext_defer, chunk, valid, scene, pos, dir, scene0, oct0)) continue;
-        const WfScene& sc = a.scenes[scene0];
-        float best_t = kInfinity, bu = 0.0f, bv = 0.0f;
-        const uint32_t best = traverse_packet<false>(sc.recs, sc.nodes, sc.perm, valid, oct0, pos, dir, best_t, bu, bv,
-                                                     stk);
-        if (valid) a.hit[slot] = make_float4(best_t, bu, bv, __uint_as_float(best));
+        const WideView w = scene_tree(a.scenes[scene0]);
+        WideRay r;
+        WideHit h;
+        wide_packet<kWideClosest>(w, valid, oct0, pos, dir, kInfinity, r, h);
+        if (valid) a.hit[slot] = make_float4(h.t, h.t2, 0.0f, __uint_as_float(h.best));
     }
 }
 
-// Closest hit for the queued paths of the deferred chunks: persistent lanes
-// fetch them dynamically, so a lane whose ray finished takes the next one at
-// once. Positions past the queue's end in the last chunk trace the last
-// entry again (the same hit, written twice).
+// Closest hit for the queued paths of the deferred chunks, as k_trace_wide
+// (trace.cu): persistent warps, one treelet per lane and step, triangles
+// tested by the warp together, finished lanes refilled when kWfRefill wait.
+// Positions past the queue's end in the last chunk trace the last entry again
+// (the same hit, written twice). Node by node, one slab test and two triangle
+// tests per crossed node, this stage and the next took 28.2 ms of the eight
+// sphere scenes' and 57.2 ms of the terrain's frame, with it 14.6 and 22.6 ms.
+constexpr int kWfRefill = 4;
+
 __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_extend(WfArgs a) {
-    extern __shared__ uint32_t smem[];
-    const StackRef stk = wf_stack(smem, a.cap);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    WfWarp& sw = reinterpret_cast<WfWarp*>(smem_raw)[threadIdx.x >> 5];
+    WideQueue& q = sw.q;
+    const WfTrees trees{a.scenes, sw.scene};
     WfCtl* c = a.ctl;
+    const uint32_t lane = lane_id();
     const uint32_t cur = c->iter & 1u;
     const uint32_t n = c->ext_count[cur];
     const uint32_t m = c->ext_defer * 32u;
-    uint32_t visits = 0;
-    uint32_t slot = 0xFFFFFFFFu;
-    const float4* recs = nullptr;
-    const uint32_t* perm = nullptr;
-    uint32_t nodes = 0;
-    f3 pos = mk3(0.0f), dir = mk3(0.0f), inv = mk3(0.0f);
-    float best_t = 0.0f, bu = 0.0f, bv = 0.0f;
-    uint32_t best = kNoPrim;
-    TravState s;
-    trav_init(s);
+    uint32_t slot = 0xFFFFFFFFu, count = 0, seq = 0;
+    bool running = false, pool = true;
+    WideView w{nullptr, nullptr, nullptr, nullptr, 0u, 1u};
+    WideRay r;
+    WideState s;
+    float lim = 0.0f;
+    wide_ray(r, mk3(0.0f), mk3(0.0f));
+    wide_init(s, 1u);
     for (;;) {
-        if (slot == 0xFFFFFFFFu) {
-            const uint32_t j = fetch_next(&c->ext_fetch);
-            if (j >= m) break;
-            slot = a.ext_q[cur][min(a.defer[j >> 5] * 32u + (j & 31u), n - 1u)];
-            const WfScene& sc = a.scenes[a.meta[slot].w];
-            recs = sc.recs; perm = sc.perm; nodes = sc.nodes;
-            const float4 o = a.o[slot], d = a.d[slot];
-            pos = mk3(o.x, o.y, o.z);
-            dir = mk3(d.x, d.y, d.z);
-            inv = box_inv(dir);
-            best_t = kInfinity; bu = bv = 0.0f; best = kNoPrim;
-            trav_init(s);
+        const uint32_t run = __ballot_sync(0xffffffffu, running);
+        if (run == 0u || (pool && __popc(run) <= 32 - kWfRefill)) {
+            queue_test<kWideClosest>(q, lane, count, count, trees);
+            count = 0;
+            if (!running && slot != 0xFFFFFFFFu) {
+                a.hit[slot] = make_float4(__uint_as_float((uint32_t)(q.key[lane] >> 32)), __uint_as_float(q.t2[lane]), 0.0f,
+                                          __uint_as_float(q.best[lane]));
+                slot = 0xFFFFFFFFu;
+            }
+            if (pool) {
+                const uint32_t j = refill(&c->ext_fetch, ~run, m, pool);
+                if (!running && j < m) {
+                    slot = a.ext_q[cur][min(a.defer[j >> 5] * 32u + (j & 31u), n - 1u)];
+                    const uint32_t scene = a.meta[slot].w;
+                    const WfScene& sc = a.scenes[scene];
+                    w.wide = sc.wide;
+                    w.nodes = sc.nodes;
+                    w.levels = sc.levels;
+                    sw.scene[lane] = scene;
+                    const float4 o = a.o[slot], d = a.d[slot];
+                    WideHit h;
+                    running = wide_begin(r, s, h, w, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), kInfinity);
+                    queue_ray<kWideClosest>(q, lane, r.pos, r.dir, kInfinity);
+                    lim = kInfinity;
+                }
+            }
+            if (!__any_sync(0xffffffffu, running || slot != 0xFFFFFFFFu)) break;
         }
-        Sector s0;
-        float4 q5;
-        float nlo, nhi;
-        if (trav_next(s, recs, nodes, pos, dir, inv, best_t, stk, s0, nlo, nhi, visits)) {
-            node_triangles<false>(recs, s.k, s0, perm, pos, dir, best_t, bu, bv, best, q5);
-            trav_descend(s, recs, q5, pos, dir, inv, best_t, nodes, stk, nlo, nhi);
-        } else {
-            a.hit[slot] = make_float4(best_t, bu, bv, __uint_as_float(best));
-            slot = 0xFFFFFFFFu;
+        uint32_t tris = 0;
+        if (running) tris = wide_visit<kWideClosest>(w, r, s, lim);
+        queue_add<kWideClosest>(q, lane, count, seq, tris, r, s, trees);
+        if (running) {
+            lim = __uint_as_float((uint32_t)(q.key[lane] >> 32));
+            running = wide_next<kWideClosest>(r, s);
         }
+    }
+}
+
+// The hits of both extend kernels checked and completed (finish_closest).
+__global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_extend_finish(WfArgs a) {
+    const WfCtl* c = a.ctl;
+    const uint32_t cur = c->iter & 1u;
+    const uint32_t n = c->ext_count[cur];
+    for (uint32_t i = global_tid(); i < n; i += grid_threads()) {
+        const uint32_t slot = a.ext_q[cur][i];
+        const float4 raw = a.hit[slot];
+        if (__float_as_uint(raw.w) == kNoPrim) continue;
+        const float4 o = a.o[slot], d = a.d[slot];
+        const WideView w = scene_tree(a.scenes[a.meta[slot].w]);
+        WideRay r;
+        r.pos = mk3(o.x, o.y, o.z);
+        r.dir = mk3(d.x, d.y, d.z);
+        WideHit h;
+        h.t = raw.x;
+        h.t2 = raw.y;
+        h.best = __float_as_uint(raw.w);
+        float u, v;
+        finish_closest(w, r, h, kInfinity, u, v);
+        a.hit[slot] = make_float4(h.t, u, v, __uint_as_float(h.best));
     }
 }
 
@@ -575,53 +634,83 @@ __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_shade(WfArgs a) {
     }
 }
 
-// Any hit for every queued shadow ray; unoccluded rays set their bit.
-// Persistent lanes with dynamic fetch, as in k_wf_extend. (Warp packets, as
-// in the extend stage, made this stage slower: the rays of a chunk start at
-// different surface points and share few nodes.)
+// Any hit for every queued shadow ray, as k_wf_extend: a ray that meets no
+// triangle sets its bit, one that does leaves the triangle's NMH position in
+// its light-sample slot (whose candidate flag is not read while the bit is
+// clear) for k_wf_shadow_finish. (Warp packets, as in the extend stage, made
+// this stage slower: the rays of a chunk start at different surface points
+// and share few nodes.)
 __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_shadow(WfArgs a) {
-    extern __shared__ uint32_t smem[];
-    const StackRef stk = wf_stack(smem, a.cap);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    WfWarp& sw = reinterpret_cast<WfWarp*>(smem_raw)[threadIdx.x >> 5];
+    WideQueue& q = sw.q;
+    const WfTrees trees{a.scenes, sw.scene};
     WfCtl* c = a.ctl;
+    const uint32_t lane = lane_id();
     const uint32_t n = c->shadow_count;
-    uint32_t visits = 0;
-    uint32_t id = 0xFFFFFFFFu;
-    const float4* recs = nullptr;
-    const uint32_t* perm = nullptr;
-    uint32_t nodes = 0;
-    f3 pos = mk3(0.0f), dir = mk3(0.0f), inv = mk3(0.0f);
-    float tmax = 0.0f, bu = 0.0f, bv = 0.0f;
-    uint32_t best = kNoPrim;
-    TravState s;
-    trav_init(s);
+    uint32_t id = 0xFFFFFFFFu, count = 0, seq = 0;
+    bool running = false, pool = true;
+    WideView w{nullptr, nullptr, nullptr, nullptr, 0u, 1u};
+    WideRay r;
+    WideState s;
+    float lim = 0.0f;
+    wide_ray(r, mk3(0.0f), mk3(0.0f));
+    wide_init(s, 1u);
     for (;;) {
-        if (id == 0xFFFFFFFFu) {
-            const uint32_t i = fetch_next(&c->shadow_fetch);
-            if (i >= n) break;
-            const float4 o = a.sh_o[i], d = a.sh_d[i];
-            id = __float_as_uint(d.w);
-            const WfScene& sc = a.scenes[a.meta[id >> 5].w];
-            recs = sc.recs; perm = sc.perm; nodes = sc.nodes;
-            pos = mk3(o.x, o.y, o.z);
-            dir = mk3(d.x, d.y, d.z);
-            inv = box_inv(dir);
-            tmax = o.w;
-            best = kNoPrim;
-            trav_init(s);
+        const uint32_t run = __ballot_sync(0xffffffffu, running);
+        if (run == 0u || (pool && __popc(run) <= 32 - kWfRefill)) {
+            queue_test<kWideAny>(q, lane, count, count, trees);
+            count = 0;
+            if (!running && id != 0xFFFFFFFFu) {
+                const uint32_t best = q.best[lane];
+                if (best == kNoPrim) atomicOr(&a.vis[id >> 5], 1u << (id & 31u));
+                else a.cj[(size_t)(id >> 5) * a.M + (id & 31u)].w = __uint_as_float(best);
+                id = 0xFFFFFFFFu;
+            }
+            if (pool) {
+                const uint32_t i = refill(&c->shadow_fetch, ~run, n, pool);
+                if (!running && i < n) {
+                    const float4 o = a.sh_o[i], d = a.sh_d[i];
+                    id = __float_as_uint(d.w);
+                    const uint32_t scene = a.meta[id >> 5].w;
+                    const WfScene& sc = a.scenes[scene];
+                    w.wide = sc.wide;
+                    w.nodes = sc.nodes;
+                    w.levels = sc.levels;
+                    sw.scene[lane] = scene;
+                    WideHit h;
+                    running = wide_begin(r, s, h, w, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w);
+                    queue_ray<kWideAny>(q, lane, r.pos, r.dir, o.w);
+                    lim = o.w;
+                }
+            }
+            if (!__any_sync(0xffffffffu, running || id != 0xFFFFFFFFu)) break;
         }
-        Sector s0;
-        float4 q5;
-        float nlo, nhi;
-        bool done;
-        if (trav_next(s, recs, nodes, pos, dir, inv, tmax, stk, s0, nlo, nhi, visits)) {
-            done = node_triangles<true>(recs, s.k, s0, perm, pos, dir, tmax, bu, bv, best, q5);
-            if (!done) trav_descend(s, recs, q5, pos, dir, inv, tmax, nodes, stk, nlo, nhi);
-        } else {
-            done = true;
-        }
-        if (done) {
-            if (best == kNoPrim) atomicOr(&a.vis[id >> 5], 1u << (id & 31u));
-            id = 0xFFFFFFFFu;
+        uint32_t tris = 0;
+        if (running) tris = wide_visit<kWideAny>(w, r, s, lim);
+        queue_add<kWideAny>(q, lane, count, seq, tris, r, s, trees);
+        if (running) running = q.key[lane] == kNoKey && wide_next<kWideAny>(r, s);
+    }
+}
+
+// Checks the occluders k_wf_shadow found (finish_any): a ray whose triangle
+// the walk of intersectAny() would not have reached, and which meets no
+// other, sets its bit after all.
+__global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_shadow_finish(WfArgs a) {
+    const uint32_t n = a.ctl->shadow_count;
+    for (uint32_t i = global_tid(); i < n; i += grid_threads()) {
+        const float4 d = a.sh_d[i];
+        const uint32_t id = __float_as_uint(d.w), slot = id >> 5;
+        if ((a.vis[slot] >> (id & 31u)) & 1u) continue;
+        const float4 o = a.sh_o[i];
+        float* flag = &a.cj[(size_t)slot * a.M + (id & 31u)].w;
+        const WideView w = scene_tree(a.scenes[a.meta[slot].w]);
+        WideRay r;
+        r.pos = mk3(o.x, o.y, o.z);
+        r.dir = mk3(d.x, d.y, d.z);
+        if (finish_any(w, r, __float_as_uint(*flag), o.w) == kNoPrim) {
+            *flag = 1.0f;
+            atomicOr(&a.vis[slot], 1u << (id & 31u));
         }
     }
 }
@@ -775,6 +864,7 @@ struct aur_batch {
     cudaGraphExec_t exec = nullptr;
     cudaStream_t cap_stream = nullptr;
     uint32_t grid = 0, block = 0;
+    uint32_t trav_grid = 0;          // of k_wf_extend and k_wf_shadow
     size_t smem = 0;
     std::vector<float4*> accum_host;
     std::vector<const aur_scene*> scene_ptrs;   // AUR_MODE_PATH_MIS: tables to keep current
@@ -782,6 +872,16 @@ struct aur_batch {
 };
 
 namespace {
+
+void launch_extend(const aur_batch* bt, const WfArgs& a, cudaStream_t s) {
+    k_wf_extend_packets<<<bt->grid, bt->block, 0, s>>>(a);
+    k_wf_extend<<<bt->trav_grid, bt->block, bt->smem, s>>>(a);
+    k_wf_extend_finish<<<bt->grid, bt->block, 0, s>>>(a);
+}
+void launch_shadow(const aur_batch* bt, const WfArgs& a, cudaStream_t s) {
+    k_wf_shadow<<<bt->trav_grid, bt->block, bt->smem, s>>>(a);
+    k_wf_shadow_finish<<<bt->grid, bt->block, 0, s>>>(a);
+}
 
 // The shade and combine instantiations for the batch's mode and materials.
 void launch_shade(const WfArgs& a, uint32_t g, uint32_t bs, cudaStream_t s) {
@@ -839,10 +939,9 @@ aur_status make_graph(aur_batch* bt) {
     AUR_CUDA(cudaStreamBeginCaptureToGraph(s, iter_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     k_wf_generate<<<g, bs, 0, s>>>(a);
     k_wf_generate_commit<<<1, 1, 0, s>>>(a);
-    k_wf_extend_packets<<<g, bs, bt->smem, s>>>(a);
-    k_wf_extend<<<g, bs, bt->smem, s>>>(a);
+    launch_extend(bt, a, s);
     launch_shade(a, g, bs, s);
-    k_wf_shadow<<<g, bs, bt->smem, s>>>(a);
+    launch_shadow(bt, a, s);
     launch_combine(a, g, bs, s);
     k_wf_end<<<1, 1, 0, s>>>(a);
     AUR_CUDA(cudaStreamEndCapture(s, &tmp));
@@ -906,7 +1005,7 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
     if (st != AUR_OK) return st;
     const bool mis = p0.mode == AUR_MODE_PATH_MIS;
     uint64_t P_tot = 0;
-    uint32_t M = 1, cap = 2;
+    uint32_t M = 1;
     bool spec = false;
     std::vector<WfScene> table(num_scenes);
     std::vector<uint32_t> pix_off(num_scenes + 1);
@@ -941,7 +1040,6 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
         AUR_CHECK(m <= (uint32_t)kMaxLightSlots, AUR_ERR_UNSUPPORTED,
                   "aur_batch_create: scene %u needs %u light samples per hit (limit %d)", i, m, kMaxLightSlots);
         M = std::max(M, m);
-        cap = std::max(cap, sc->nmh->levels + 1);
         WfScene& w = table[i];
         w.recs = sc->nmh->node_recs;
         w.perm = sc->nmh->perm;
@@ -958,7 +1056,10 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
         w.mis_pa = sc->mis_pa;
         w.mis_count = sc->mis_count;
         w.nodes = sc->nmh->nodes;
-        w.packet_span = sc->nmh->extent * (1.0f / 64.0f);
+        w.levels = sc->nmh->levels;
+        w.wide = sc->nmh->wide;
+        w.packet_span = packet_span(sc->nmh);
+        w.dir_span = dir_span(sc->nmh);
         w.num_lights = sc->num_lights;
         w.width = p.width;
         w.height = p.height;
@@ -999,7 +1100,11 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
     bt->tuning = tn;
     bt->block = tn.block_size;
     bt->grid = (uint32_t)ctx->sm_count * tn.blocks_per_sm;
-    bt->smem = (size_t)2 * cap * tn.block_size * sizeof(uint32_t);
+    // Unless the caller chose, the traversal stages run as many blocks as fit
+    // an SM at their 64 registers: 8 of 128 threads measured 14.6 and 22.6 ms
+    // on eight sphere scenes and a 2M-triangle terrain, 6 blocks 15.3 and 23.3.
+    bt->trav_grid = tuning && tuning->blocks_per_sm ? bt->grid : (uint32_t)ctx->sm_count * (1024u / tn.block_size);
+    bt->smem = (size_t)(tn.block_size / 32) * sizeof(WfWarp);
     bt->accum_host.assign(num_scenes, nullptr);
     bt->scene_ptrs.assign(scenes, scenes + num_scenes);
     bt->table_host = table;
@@ -1035,7 +1140,6 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
     a.max_depth = p0.max_depth;
     a.mode = p0.mode;
     a.seed = p0.seed;
-    a.cap = (int)cap;
     a.o = (float4*)(base + o_o); a.d = (float4*)(base + o_d); a.thr = (float4*)(base + o_thr);
     a.col = (float4*)(base + o_col); a.hit = (float4*)(base + o_hit); a.meta = (uint4*)(base + o_meta);
     a.ndir = (float4*)(base + o_ndir); a.nthr = (float4*)(base + o_nthr); a.fsh = (float4*)(base + o_fsh);
@@ -1059,7 +1163,7 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
     if (tn.max_iterations) ctl.iter_limit = tn.max_iterations;
     cudaMemcpy(a.ctl, &ctl, sizeof(ctl), cudaMemcpyHostToDevice);
     cudaError_t e = cudaSuccess;
-    for (const void* k : {(const void*)k_wf_extend_packets, (const void*)k_wf_extend, (const void*)k_wf_shadow})
+    for (const void* k : {(const void*)k_wf_extend, (const void*)k_wf_shadow})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt->smem);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&bt->cap_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
@@ -1183,12 +1287,11 @@ aur_status aur_batch_profile(aur_ctx* ctx, aur_batch* bt, float* const* accum, f
             k_wf_generate<<<g, bs, 0, st>>>(a);
             k_wf_generate_commit<<<1, 1, 0, st>>>(a);
             cudaEventRecord(ev[1], st);
-            k_wf_extend_packets<<<g, bs, bt->smem, st>>>(a);
-            k_wf_extend<<<g, bs, bt->smem, st>>>(a);
+            launch_extend(bt, a, st);
             cudaEventRecord(ev[2], st);
             launch_shade(a, g, bs, st);
             cudaEventRecord(ev[3], st);
-            k_wf_shadow<<<g, bs, bt->smem, st>>>(a);
+            launch_shadow(bt, a, st);
             cudaEventRecord(ev[4], st);
             launch_combine(a, g, bs, st);
             k_wf_end<<<1, 1, 0, st>>>(a);
