@@ -32,6 +32,7 @@
 // table weighs triangles by the shader's scalar `emission` times area
 // (emitter.cu's weight), not by its emission colour.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -44,9 +45,11 @@ namespace aur {
 namespace {
 
 constexpr int kAdjThreads = 128;
-// The replay kernel is compiled for 8 resident blocks per SM (at most 64
-// registers): 24 % faster than its free 150-160 registers (3 blocks).
-constexpr int kAdjBlocksPerSm = 8;
+// The replay kernel is compiled for 14 resident blocks per SM (at most 36
+// registers, spills served by L1): its lanes diverge and it waits on latency,
+// so more warps pay for the spills. 256x256, 16 samples of the 4130-triangle
+// box: 6.1 ms at 8 blocks, 5.9 at 10, 5.8 at 12, 5.3 at 14 and 16.
+constexpr int kAdjBlocksPerSm = 14;
 constexpr uint32_t kSharedLights = 64;
 
 // Per-unit-colour radiance of a light sample (Lr = color * s), light.cuh:228-259.
@@ -101,13 +104,12 @@ __device__ __forceinline__ void add_shader_grad(float* __restrict__ d, uint32_t 
 // whether a diffuse bounce follows the hit (both for AUR_MODE_PATH_MIS).
 // With d_emission, the emission gradients of the hit's own shader si and of
 // the emitter sample's shader are added too.
-template <bool kMis>
+template <bool kMis, typename Trav>
 __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader* sh, const Bsdf& b, const f3& f,
                                           const f3& position, const f3& wo, float ew, bool bounce, uint32_t seed,
                                           uint32_t scene, uint32_t pixel, uint32_t sample, uint32_t rix, const f3& thr,
                                           const f3& g, float* __restrict__ d_light, f3& gl0, f3& Dp,
-                                          float* __restrict__ d_emission, uint32_t si, const StackRef& stk,
-                                          uint32_t& visits, uint32_t* err) {
+                                          float* __restrict__ d_emission, uint32_t si, const Trav& trav, uint32_t* err) {
     f3 Li = kMis ? from(sh->emission_color) * ew : from(sh->emission_color);
     if (d_emission) add_shader_grad(d_emission, si, kMis ? (g * thr) * ew : g * thr);
     Dp = mk3(0.0f);   // direct light per unit Lambert colour
@@ -124,9 +126,8 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
             f3 wdir; float wt, pdf;
             const f3 Ls = sample_light(L, position, seed, scene, pixel, sample, rix, 0u, wdir, wt, pdf);
             if (pdf > 0.0f && !zero(Ls)) {
-                float du = 0.0f, dv = 0.0f;
                 if (!zero(f) &&
-                    traverse<true>(sc.recs, sc.nodes, sc.perm, position, wdir, wt, du, dv, stk, visits, err) == kNoPrim) {
+                    !occluded(sc, trav, position, wdir, wt)) {
                     const float cs = fmaxf(0.0f, dot(wdir, b.N));
                     Li = Li + f * Ls * cs;
                     Dp = Dp + Ls * (kInvPi * cs);
@@ -146,9 +147,8 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
                                                         sample, rix)
                                     : area_bsdf_sample(q, i, (uint32_t)j, b, f, position, wo, seed, scene, pixel,
                                                        sample, rix);
-                        float du = 0.0f, dv = 0.0f, tt = ss.tmax;
-                        if (ss.cand && traverse<true>(sc.recs, sc.nodes, sc.perm, ss.o, ss.d, tt, du, dv, stk,
-                                                      visits, err) == kNoPrim) {
+                        const float tt = ss.tmax;
+                        if (ss.cand && !occluded(sc, trav, ss.o, ss.d, tt)) {
                             Ls = Ls + ss.c;
                             accp = accp + ss.e * (ss.geo * kInvPi);
                             accl = accl + f * (L.intensity * ss.geo);
@@ -173,9 +173,8 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
                 wpos.z += kEpsilon * wdir.z;
                 wt += kEpsilon;
                 if (lpdf > 0.0f && !zero(Lr)) {
-                    float du = 0.0f, dv = 0.0f;
-                    if (!zero(f) &&
-                        traverse<true>(sc.recs, sc.nodes, sc.perm, wpos, wdir, wt, du, dv, stk, visits, err) == kNoPrim) {
+                        if (!zero(f) &&
+                        !occluded(sc, trav, wpos, wdir, wt)) {
                         const float cs = fmaxf(0.0f, dot(wdir, b.N));
                         acc = acc + f * Lr * cs;
                         accp = accp + Lr * (kInvPi * cs);
@@ -200,9 +199,8 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
     if (kMis) {   // the emitter sample (direct_light_mis)
         const ShadowSample ss =
             emitter_shadow_sample(sc, b, f, position, wo, bounce, seed, scene, pixel, sample, rix);
-        float du = 0.0f, dv = 0.0f, tt = ss.tmax;
-        const bool vis = ss.cand && traverse<true>(sc.recs, sc.nodes, sc.perm, ss.o, ss.d, tt, du, dv, stk,
-                                                   visits, err) == kNoPrim;
+        const float tt = ss.tmax;
+        const bool vis = ss.cand && !occluded(sc, trav, ss.o, ss.d, tt);
         Li = Li + (vis ? ss.c : mk3(0.0f));
         if (vis) Dp = Dp + ss.e * (ss.geo * kInvPi);
         if (d_emission && vis) add_shader_grad(d_emission, ss.esi, (g * thr) * (f * ss.geo));
@@ -226,11 +224,11 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
 // colour and in the light colour. One pass replaces a primal pass (each
 // sample's radiance) plus a replay: 29.3 -> 21.1 ms on the differentiable
 // workload (256x256, 64 spp, path mode).
-template <bool kMis>
+template <bool kMis, typename Trav>
 __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t mode, uint32_t seed, uint32_t scene,
-                             uint32_t pixel, uint32_t sample, const PathRay& primary, const StackRef& stk,
+                             uint32_t pixel, uint32_t sample, const PathRay& primary, const Trav& trav,
                              const f3& g, float* __restrict__ d_diffuse, float* __restrict__ d_light,
-                             float* __restrict__ d_emission, f3& gl0, uint32_t& visits, uint32_t* err) {
+                             float* __restrict__ d_emission, f3& gl0, uint32_t* err) {
     struct Marker {
         f3 col0, c1;          // colour before the subtree, the bouncing vertex's Lambert colour
         const aur_shader* sh;
@@ -260,7 +258,7 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
         PathRay ray = stack[--sp];
         const uint32_t rix = ray_index++;
         float t = kInfinity, u = 0.0f, v = 0.0f;
-        const uint32_t tri = traverse<false>(sc.recs, sc.nodes, sc.perm, ray.pos, ray.dir, t, u, v, stk, visits, err);
+        const uint32_t tri = closest_hit(sc, trav, ray.pos, ray.dir, t, u, v);
         if (tri == kNoPrim) continue;
         const f3 position = ray.pos + (ray.dir * t);
         const f3 wo = -ray.dir;
@@ -280,7 +278,7 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
             continue_ray<kMis>(sh, b, cur, position, wo, path, depth, maxd, seed, scene, pixel, sample, rix);
         f3 Dp;
         const f3 Li = direct_grad<kMis>(sc, sh, b, f, position, wo, ew, bounce_follows, seed, scene, pixel, sample, rix,
-                                        cur.thr, g, d_light, gl0, Dp, d_emission, si, stk, visits, err);
+                                        cur.thr, g, d_light, gl0, Dp, d_emission, si, trav, err);
         add_diffuse_grad(d_diffuse, si, sh, g * (cur.thr * Dp));
         col = col + Li * cur.thr;
         for (int q = 0; q < kc.n; ++q) {
@@ -299,17 +297,8 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
     while (nm > 0) close(mk[--nm]);
 }
 
-__device__ __forceinline__ StackRef adj_stack(uint32_t* smem, int cap) {
-    StackRef stk;
-    stk.lo = reinterpret_cast<float*>(smem) + threadIdx.x;
-    stk.hi = reinterpret_cast<float*>(smem + cap * kAdjThreads) + threadIdx.x;
-    stk.stride = kAdjThreads;
-    stk.cap = cap;
-    return stk;
-}
-
 // Replay kernel: one thread per camera sample of samples [s0, s0 + nb).
-template <bool kMis>
+template <bool kMis, bool kTiny>
 __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) k_adj_replay(SceneView sc, aur_camera cam,
                                                                             aur_render_params p, uint32_t s0,
                                                                             uint32_t nb,
@@ -317,11 +306,10 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) k_adj_replay(Sce
                                                                             float* __restrict__ d_diffuse,
                                                                             float* __restrict__ d_light,
                                                                             float* __restrict__ d_emission,
-                                                                            uint32_t* __restrict__ err, int cap) {
-    extern __shared__ uint32_t smem[];
-    const StackRef stk = adj_stack(smem, cap);
+                                                                            uint32_t* __restrict__ err) {
+    const auto trav = make_trav<kTiny>(sc);
+    __shared__ float s_light[3 * kSharedLights];
     // light gradients are reduced in shared memory first (one light is hit by every sample)
-    float* s_light = reinterpret_cast<float*>(smem + 2 * cap * kAdjThreads);
     const bool shared_lights = sc.num_lights <= kSharedLights;
     if (shared_lights)
         for (uint32_t i = threadIdx.x; i < 3 * sc.num_lights; i += kAdjThreads) s_light[i] = 0.0f;
@@ -336,9 +324,8 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) k_adj_replay(Sce
         const float4 di = d_image[pix];
         const float w = 1.0f / (float)p.spp;
         const f3 g = mk3(di.x * w, di.y * w, di.z * w);
-        uint32_t visits = 0;
-        replay_stack<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, stk, g, d_diffuse,
-                           shared_lights ? s_light : d_light, d_emission, gl0, visits, err);
+        replay_stack<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, d_diffuse,
+                           shared_lights ? s_light : d_light, d_emission, gl0, err);
     }
     // light 0: warp sum, then one shared atomic per warp
 #pragma unroll
@@ -393,21 +380,18 @@ aur_status aur_render_adjoint(aur_ctx* ctx, const aur_scene* scene, const aur_ca
     if (s1 == s0) return AUR_OK;
     const uint64_t P = (uint64_t)p.width * p.height;
     const uint32_t batch = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(s1 - s0, (1ull << 24) / P));
-    const int cap = (int)scene->nmh->levels + 1;
-    const size_t smem = (size_t)2 * cap * kAdjThreads * sizeof(uint32_t) + 3 * kSharedLights * sizeof(float);
-    AUR_CUDA(cudaFuncSetAttribute(k_adj_replay<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    AUR_CUDA(cudaFuncSetAttribute(k_adj_replay<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const SceneView sv = scene_view(scene);
     const float4* di = (const float4*)d_image;
     for (uint32_t s = s0; s < s1; s += batch) {
         const uint32_t nb = std::min(batch, s1 - s);
         const uint32_t grid = cdiv(P * nb, kAdjThreads);
-        if (mis)
-            k_adj_replay<true><<<grid, kAdjThreads, smem, ctx->stream>>>(sv, *camera, p, s, nb, di, d_diffuse,
-                                                                        d_light_color, d_emission, ctx->d_flags, cap);
-        else
-            k_adj_replay<false><<<grid, kAdjThreads, smem, ctx->stream>>>(sv, *camera, p, s, nb, di, d_diffuse,
-                                                                         d_light_color, d_emission, ctx->d_flags, cap);
+        auto go = [&](auto m, auto tiny) {
+            k_adj_replay<m.value, tiny.value><<<grid, kAdjThreads, 0, ctx->stream>>>(
+                sv, *camera, p, s, nb, di, d_diffuse, d_light_color, d_emission, ctx->d_flags);
+        };
+        const bool tiny = scene->nmh->count <= kTinyTris;
+        if (mis) tiny ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+        else tiny ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
     }
     AUR_CUDA(cudaGetLastError());
     return AUR_OK;

@@ -11,12 +11,14 @@
 
 #include "aur_math.cuh"
 #include "aur_traverse.cuh"
+#include "aur_wide.cuh"
 
 namespace aur {
 
 struct SceneView {
     const float4* recs;
-    uint32_t nodes;
+    const uint4* wide;
+    uint32_t nodes, levels;
     const uint32_t* perm;
     const float* normals;      // NMH order, 9 floats per triangle
     const uint16_t* sids;      // NMH order, 1-based
@@ -35,6 +37,78 @@ struct SceneView {
 };
 
 SceneView scene_view(const aur_scene* sc);
+
+// How the integrators' kernels trace: over the treelets, each lane on its own
+// (the warp working together on its rays, as in the trace kernels, makes
+// every lane wait for the slowest of 32 at each trace: 2.5 ms against 1.9 ms
+// on a 200k-triangle sphere scene), or, where the scene has at most
+// kTinyTris triangles, by testing them all from shared memory.
+struct TreeTrav {
+    static constexpr bool kTiny = false;
+};
+struct TinyTrav {
+    static constexpr bool kTiny = true;
+    const float4* tris;    // stage_tiny's triangles
+    uint32_t count;
+};
+
+// The kernel's way to trace: in a kTiny kernel, its scene's triangles staged
+// in shared memory by the whole block.
+template <bool kTiny>
+__device__ __forceinline__ auto make_trav(const SceneView& sc) {
+    if constexpr (kTiny) {
+        __shared__ float4 s_tri[3 * kTinyTris];
+        stage_tiny(s_tri, sc.verts, sc.perm, 2u * sc.nodes);
+        __syncthreads();
+        return TinyTrav{s_tri, 2u * sc.nodes};
+    } else {
+        return TreeTrav{};
+    }
+}
+
+__device__ __forceinline__ WideView tree_of(const SceneView& sc) {
+    return WideView{sc.recs, sc.wide, sc.perm, sc.verts, sc.nodes, sc.levels};
+}
+
+// Closest hit over (Epsilon, t): the NMH position (kNoPrim: none), t, u, v.
+template <typename Trav>
+__device__ __forceinline__ uint32_t closest_hit(const SceneView& sc, const Trav& trav, const f3& pos, const f3& dir,
+                                                float& t, float& u, float& v) {
+    const WideView w = tree_of(sc);
+    WideRay r;
+    WideHit h;
+    const float tmax = t;
+    if constexpr (Trav::kTiny) {
+        r.pos = pos;
+        r.dir = dir;
+        tiny_closest(trav.tris, trav.count, pos, dir, tmax, h);
+    } else {
+        WideState s;
+        if (wide_begin(r, s, h, w, pos, dir, tmax))
+            while (wide_step<kWideClosest>(w, r, s, h)) {}
+    }
+    finish_closest(w, r, h, tmax, u, v);
+    if (h.best != kNoPrim) t = h.t;
+    return h.best;
+}
+
+// True when a triangle is hit over (Epsilon, tmax).
+template <typename Trav>
+__device__ __forceinline__ bool occluded(const SceneView& sc, const Trav& trav, const f3& pos, const f3& dir, float tmax) {
+    const WideView w = tree_of(sc);
+    WideRay r;
+    WideHit h;
+    if constexpr (Trav::kTiny) {
+        r.pos = pos;
+        r.dir = dir;
+        h.best = tiny_any(trav.tris, trav.count, pos, dir, tmax);
+    } else {
+        WideState s;
+        if (wide_begin(r, s, h, w, pos, dir, tmax))
+            while (wide_step<kWideAny>(w, r, s, h)) {}
+    }
+    return finish_any(w, r, h.best, tmax) != kNoPrim;
+}
 
 // Texture units of the reference (texunit.cuh:11-18): normalised
 // coordinates, wrap addressing, linear filtering, RGBA8 read as byte / 255.
@@ -447,10 +521,11 @@ __device__ __forceinline__ ShadowSample emitter_shadow_sample(const SceneView& s
 // sample, the emitter's) is traced at one call site: the loop walks light
 // i, sample j and the strategy, so the kernel holds one inlined copy of the
 // any-hit traversal for all of them instead of four.
+template <typename Trav>
 __device__ __forceinline__ f3 direct_light_mis(const SceneView& sc, const aur_shader* sh, const Bsdf& b,
                                                const f3& position, const f3& wo, float ew, bool bounce,
                                                uint32_t seed, uint32_t scene, uint32_t pixel, uint32_t sample,
-                                               uint32_t rix, const StackRef& stk, uint32_t& visits, uint32_t* err) {
+                                               uint32_t rix, const Trav& trav, uint32_t* err) {
     f3 Li = from(sh->emission_color) * ew;
     const f3 f = bsdf_f(b);
     const uint32_t nl = sc.num_lights;
@@ -504,9 +579,7 @@ __device__ __forceinline__ f3 direct_light_mis(const SceneView& sc, const aur_sh
             emitter = true;
             ++i;
         }
-        float du = 0.0f, dv = 0.0f;
-        const bool vis =
-            s.cand && traverse<true>(sc.recs, sc.nodes, sc.perm, s.o, s.d, s.tmax, du, dv, stk, visits, err) == kNoPrim;
+        const bool vis = s.cand && !occluded(sc, trav, s.o, s.d, s.tmax);
         if (to_ls) {
             if (vis) Ls = Ls + s.c;
         } else if (emitter) {
@@ -529,13 +602,12 @@ __device__ __forceinline__ f3 direct_light_mis(const SceneView& sc, const aur_sh
 // reference's order (monteCarloRaytracer.cu:42-52, radiance.cuh:13-80).
 // kMis: direct_light_mis; `bounce` says whether a diffuse bounce follows
 // this hit.
-template <bool kMis>
+template <bool kMis, typename Trav>
 __device__ __forceinline__ f3 direct_light(const SceneView& sc, const aur_shader* sh, const Bsdf& b, const f3& position,
                                            const f3& wo, float ew, bool bounce, uint32_t seed, uint32_t scene,
-                                           uint32_t pixel, uint32_t sample, uint32_t rix, const StackRef& stk,
-                                           uint32_t& visits, uint32_t* err) {
+                                           uint32_t pixel, uint32_t sample, uint32_t rix, const Trav& trav, uint32_t* err) {
     if constexpr (kMis)
-        return direct_light_mis(sc, sh, b, position, wo, ew, bounce, seed, scene, pixel, sample, rix, stk, visits, err);
+        return direct_light_mis(sc, sh, b, position, wo, ew, bounce, seed, scene, pixel, sample, rix, trav, err);
     f3 Li = from(sh->emission_color);
     for (uint32_t i = 0; i < sc.num_lights; ++i) {
         const aur_light& L = sc.lights[i];
@@ -546,9 +618,8 @@ __device__ __forceinline__ f3 direct_light(const SceneView& sc, const aur_shader
             const f3 Ls = sample_light(L, position, seed, scene, pixel, sample, rix, 0u, wdir, wt, pdf);
             if (pdf > 0.0f && !zero(Ls)) {
                 const f3 f = bsdf_f(b);
-                float du = 0.0f, dv = 0.0f;
                 if (!zero(f) &&
-                    traverse<true>(sc.recs, sc.nodes, sc.perm, position, wdir, wt, du, dv, stk, visits, err) == kNoPrim)
+                    !occluded(sc, trav, position, wdir, wt))
                     Li = Li + f * Ls * fmaxf(0.0f, dot(wdir, b.N));
             }
         } else {
@@ -567,9 +638,8 @@ __device__ __forceinline__ f3 direct_light(const SceneView& sc, const aur_shader
                 wt += kEpsilon;
                 if (lpdf > 0.0f && !zero(Lr)) {
                     const f3 f = bsdf_f(b);
-                    float du = 0.0f, dv = 0.0f;
-                    if (!zero(f) &&
-                        traverse<true>(sc.recs, sc.nodes, sc.perm, wpos, wdir, wt, du, dv, stk, visits, err) == kNoPrim)
+                        if (!zero(f) &&
+                        !occluded(sc, trav, wpos, wdir, wt))
                         Ls = Ls + f * Lr * fmaxf(0.0f, dot(wdir, b.N));
                 }
                 acc = acc + Ls;
@@ -671,10 +741,10 @@ __device__ __forceinline__ Continuation continue_ray(const aur_shader* sh, const
 
 // Integrates one camera ray. RNG key: (seed, scene_id) x (pixel, sample,
 // ray index within the sample, slot). kMis: mode is AUR_MODE_PATH_MIS.
-template <bool kMis = false>
+template <bool kMis, typename Trav>
 __device__ __forceinline__ SampleResult integrate(const SceneView& sc, uint32_t max_depth, uint32_t mode,
                                                   uint32_t seed, uint32_t scene, uint32_t pixel, uint32_t sample,
-                                                  const PathRay& primary, const StackRef& stk, uint32_t& visits,
+                                                  const PathRay& primary, const Trav& trav,
                                                   uint32_t* err) {
     PathRay stack[AUR_MAX_DEPTH + 2];
     int sp = 0;
@@ -693,7 +763,7 @@ __device__ __forceinline__ SampleResult integrate(const SceneView& sc, uint32_t 
         PathRay ray = stack[--sp];
         const uint32_t rix = ray_index++;
         float t = kInfinity, u = 0.0f, v = 0.0f;
-        const uint32_t tri = traverse<false>(sc.recs, sc.nodes, sc.perm, ray.pos, ray.dir, t, u, v, stk, visits, err);
+        const uint32_t tri = closest_hit(sc, trav, ray.pos, ray.dir, t, u, v);
         if (tri == kNoPrim) continue;
         res.any_hit = true;
         const f3 position = ray.pos + (ray.dir * t);
@@ -706,7 +776,7 @@ __device__ __forceinline__ SampleResult integrate(const SceneView& sc, uint32_t 
         const bool specular = refl > 0.0f || trans > 0.0f;
         const float ew = kMis ? emission_weight(sc, tri, ray.dir, t, ray.pdf) : 1.0f;
         const f3 Li = direct_light<kMis>(sc, sh, b, position, wo, ew, !specular && depth + 1 <= maxd, seed, scene,
-                                         pixel, sample, rix, stk, visits, err);
+                                         pixel, sample, rix, trav, err);
         const Continuation k =
             continue_ray<kMis>(sh, b, ray, position, wo, path, depth, maxd, seed, scene, pixel, sample, rix);
         for (int q = 0; q < k.n; ++q) {
@@ -720,11 +790,10 @@ __device__ __forceinline__ SampleResult integrate(const SceneView& sc, uint32_t 
 // The same estimator for scenes without specular shaders: one ray in flight
 // per sample, no ray stack (a Lambert hit spawns at most the diffuse bounce).
 // Same operations in the same order as integrate().
-template <bool kMis = false>
+template <bool kMis, typename Trav>
 __device__ __forceinline__ SampleResult integrate_diffuse(const SceneView& sc, uint32_t max_depth, uint32_t mode,
                                                           uint32_t seed, uint32_t scene, uint32_t pixel,
-                                                          uint32_t sample, const PathRay& primary, const StackRef& stk,
-                                                          uint32_t& visits, uint32_t* err) {
+                                                          uint32_t sample, const PathRay& primary, const Trav& trav, uint32_t* err) {
     SampleResult res;
     res.color = mk3(0.0f);
     res.any_hit = false;
@@ -737,7 +806,7 @@ __device__ __forceinline__ SampleResult integrate_diffuse(const SceneView& sc, u
     uint32_t depth = 0;
     for (uint32_t rix = 0;; ++rix) {
         float t = kInfinity, u = 0.0f, v = 0.0f;
-        const uint32_t tri = traverse<false>(sc.recs, sc.nodes, sc.perm, pos, dir, t, u, v, stk, visits, err);
+        const uint32_t tri = closest_hit(sc, trav, pos, dir, t, u, v);
         if (tri == kNoPrim) break;
         res.any_hit = true;
         const f3 position = pos + (dir * t);
@@ -748,7 +817,7 @@ __device__ __forceinline__ SampleResult integrate_diffuse(const SceneView& sc, u
         const Bsdf b = get_bsdf(sc, sh, tri, u, v);
         const float ew = kMis ? emission_weight(sc, tri, dir, t, prev_pdf) : 1.0f;
         const f3 Li = direct_light<kMis>(sc, sh, b, position, wo, ew, depth + 1 <= max_depth, seed, scene, pixel,
-                                         sample, rix, stk, visits, err);
+                                         sample, rix, trav, err);
         res.color = res.color + Li * thr;
         if (!path) break;
         if (++depth > max_depth) break;

@@ -580,6 +580,70 @@ __device__ __forceinline__ void wide_warp(const WideView& w, WideQueue& q, bool 
 }
 #endif  // __CUDACC__
 
+// ------------------------------------------------------------ a few triangles
+// An NMH of at most kTinyTris triangles has no use for a tree: every lane
+// tests every triangle, staged in shared memory and read by the whole warp at
+// one address, so no lane waits for another's path and no load waits for a
+// node. (1M rays, 100 triangles: 0.20 ms so, 0.20 ms over the treelets; 34:
+// 0.10 ms against 0.19 ms.)
+constexpr uint32_t kTinyTris = 64;
+
+#ifdef __CUDACC__
+// Stages `count` triangles as (v1, prim id), e1, e2: 3 * count float4. The
+// whole block calls it, and synchronizes before reading them.
+__device__ __forceinline__ void stage_tiny(float4* __restrict__ s_tri, const float* __restrict__ verts,
+                                           const uint32_t* __restrict__ perm, uint32_t count) {
+    for (uint32_t j = threadIdx.x; j < count; j += blockDim.x) {
+        const float* q = verts + (size_t)j * 9;
+        s_tri[3 * j] = make_float4(q[0], q[3], q[6], __uint_as_float(perm[j]));
+        s_tri[3 * j + 1] = make_float4(q[1] - q[0], q[4] - q[3], q[7] - q[6], 0.0f);
+        s_tri[3 * j + 2] = make_float4(q[2] - q[0], q[5] - q[3], q[8] - q[6], 0.0f);
+    }
+}
+
+__device__ __forceinline__ bool tiny_tri(const float4* __restrict__ tris, uint32_t j, const f3& pos, const f3& dir,
+                                         float& t, uint32_t& id) {
+    const float4 a = tris[3 * j], b = tris[3 * j + 1], c = tris[3 * j + 2];
+    float u, v;
+    id = __float_as_uint(a.w);
+    return intersect_tri(pos, dir, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), mk3(c.x, c.y, c.z), u, v, t) && t > kEpsilon;
+}
+
+__device__ __forceinline__ void tiny_closest(const float4* __restrict__ tris, uint32_t count, const f3& pos,
+                                             const f3& dir, float tmax, WideHit& h) {
+    h.t = h.t2 = tmax;
+    h.best = kNoPrim;
+    uint32_t best_id = 0;
+    for (uint32_t j = 0; j < count; ++j) {
+        float t;
+        uint32_t id;
+        if (!tiny_tri(tris, j, pos, dir, t, id)) continue;
+        if (t < h.t) {
+            h.t2 = h.t;
+            h.t = t;
+            h.best = j;
+            best_id = id;
+        } else {
+            if (t == h.t && h.best != kNoPrim && id < best_id) {
+                h.best = j;
+                best_id = id;
+            }
+            h.t2 = fminf(h.t2, t);
+        }
+    }
+}
+
+__device__ __forceinline__ uint32_t tiny_any(const float4* __restrict__ tris, uint32_t count, const f3& pos,
+                                             const f3& dir, float tmax) {
+    for (uint32_t j = 0; j < count; ++j) {
+        float t;
+        uint32_t id;
+        if (tiny_tri(tris, j, pos, dir, t, id) && t < tmax) return j;
+    }
+    return kNoPrim;
+}
+#endif  // __CUDACC__
+
 // ------------------------------------------------------------ the checks
 // intersect() visits a triangle's node when the ray's range, clipped by the
 // slab of every node from the root down to it (ray.cuh:225-237), is not empty

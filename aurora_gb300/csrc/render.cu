@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "aur_integrate.cuh"
@@ -19,49 +20,38 @@ namespace aur {
 namespace {
 
 constexpr int kRenderThreads = 128;
-// The fused sample kernel is compiled for 10 resident blocks per SM (at most
-// 51 registers, a few hundred bytes of spills served by L1): measured 19 %
-// faster than its free 128 registers, which allowed 4 blocks. The per-tile
-// kernel (k_raytrace_mc) runs grids of one 65,536-ray tile, too small for
-// occupancy to matter, and is left unconstrained (a cap made it slower).
-constexpr int kRenderBlocksPerSm = 10;
-// The MIS instantiations carry more live state (two strategies per light
-// sample, the emitter sample): 8 blocks per SM (64 registers) measured 9-17 %
-// faster than 10 or 12, and 4-9 % faster than 6.
-constexpr int kRenderBlocksPerSmMis = 8;
+// Resident blocks per SM that the fused sample kernel is compiled for: its
+// lanes diverge, so what helps is more warps to switch between, even at the
+// price of spills. Measured among 4 to 16: tiny scenes, path mode 1.16-1.30 ms
+// at 4 to 10 and 1.14 at 14 (256x256 box, 16 samples); MIS 1.50-1.59 and 1.44
+// (301x233 emissive box, 9 samples); trees, path mode 1.88 at 8, 1.91 at 6 and
+// 10, 1.94 at 14 (200k-triangle spheres); MIS 2.41 at 6 to 8, 2.35 at 14
+// (4130-triangle box). The per-tile kernel (k_raytrace_mc) runs grids of one
+// 65,536-ray tile, too small for occupancy to matter, and is left
+// unconstrained (a cap made it slower).
+constexpr int render_blocks(bool mis, bool tiny) { return mis || tiny ? 14 : 8; }
 
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 const char kAccumMagic[8] = {'A', 'U', 'R', 'A', 'C', 'C', '1', '\0'};
 
-__device__ __forceinline__ StackRef stack_ref(uint32_t* smem, int cap) {
-    StackRef s;
-    s.lo = reinterpret_cast<float*>(smem) + threadIdx.x;
-    s.hi = reinterpret_cast<float*>(smem + cap * blockDim.x) + threadIdx.x;
-    s.stride = blockDim.x;
-    s.cap = cap;
-    return s;
-}
-
 // colors[b * P + p] = (rgb, hit) of sample s0 + b at pixel p. kGeneric
 // selects the integrator with the specular ray stack, kMis the
 // AUR_MODE_PATH_MIS estimator.
-template <bool kGeneric, bool kMis>
-__global__ void __launch_bounds__(kRenderThreads, kMis ? kRenderBlocksPerSmMis : kRenderBlocksPerSm) k_render_samples(SceneView sc, aur_camera cam, aur_render_params p,
-                                                                   uint32_t s0, uint32_t nb, float4* __restrict__ colors,
-                                                                   uint32_t* __restrict__ err, int cap) {
-    extern __shared__ uint32_t smem[];
-    const StackRef stk = stack_ref(smem, cap);
+template <bool kGeneric, bool kMis, bool kTiny>
+__global__ void __launch_bounds__(kRenderThreads, render_blocks(kMis, kTiny))
+    k_render_samples(SceneView sc, aur_camera cam, aur_render_params p, uint32_t s0, uint32_t nb,
+                     float4* __restrict__ colors, uint32_t* __restrict__ err) {
+    const auto trav = make_trav<kTiny>(sc);
     const uint64_t P = (uint64_t)p.width * p.height;
     const uint64_t t = (uint64_t)blockIdx.x * kRenderThreads + threadIdx.x;
     if (t >= P * nb) return;
     const uint32_t pix = (uint32_t)(t % P);
     const uint32_t s = s0 + (uint32_t)(t / P);
     const PathRay r = camera_ray(cam, p.width, p.height, pix % p.width, pix / p.width, s, p.spp);
-    uint32_t visits = 0;
     const SampleResult res =
-        kGeneric ? integrate<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, stk, visits, err)
-                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, stk, visits, err);
+        kGeneric ? integrate<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, err)
+                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, err);
     colors[t] = make_float4(res.color.x, res.color.y, res.color.z, res.any_hit ? 1.0f : 0.0f);
 }
 
@@ -101,14 +91,13 @@ __global__ void k_generate_rays(uint32_t W, uint32_t H, uint32_t sample, uint32_
 }
 
 // cudaRaytraceKernel (monteCarloRaytracer.cu:90-113) on caller-provided rays.
-template <bool kGeneric, bool kMis>
+template <bool kGeneric, bool kMis, bool kTiny>
 __global__ void __launch_bounds__(kRenderThreads) k_raytrace_mc(SceneView sc, aur_render_params p, uint32_t sample,
                                                                 uint32_t offset, uint32_t num,
                                                                 const aur_path_ray* __restrict__ rays,
                                                                 aur_hitpoint* __restrict__ hits,
-                                                                uint32_t* __restrict__ err, int cap) {
-    extern __shared__ uint32_t smem[];
-    const StackRef stk = stack_ref(smem, cap);
+                                                                uint32_t* __restrict__ err) {
+    const auto trav = make_trav<kTiny>(sc);
     const uint32_t t = blockIdx.x * kRenderThreads + threadIdx.x;
     if (t >= num) return;
     const uint32_t id = offset + t;
@@ -120,11 +109,9 @@ __global__ void __launch_bounds__(kRenderThreads) k_raytrace_mc(SceneView sc, au
     r.eta = in.eta;
     r.thr = mk3(in.weight);
     r.pdf = 0.0f;
-    uint32_t visits = 0;
     const SampleResult res =
-        kGeneric ? integrate<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, id, sample, r, stk, visits, err)
-                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, id, sample, r, stk, visits,
-                                           err);
+        kGeneric ? integrate<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, id, sample, r, trav, err)
+                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, id, sample, r, trav, err);
     aur_hitpoint h = hits[id];
     h.color = to(from(h.color) + res.color);
     if (res.any_hit) {
@@ -202,7 +189,9 @@ __global__ void k_filter_pixels(uint32_t width, aur_rect r, const float4* __rest
 SceneView scene_view(const aur_scene* sc) {
     SceneView v;
     v.recs = sc->nmh->node_recs;
+    v.wide = sc->nmh->wide;
     v.nodes = sc->nmh->nodes;
+    v.levels = sc->nmh->levels;
     v.perm = sc->nmh->perm;
     v.normals = sc->normals;
     v.sids = sc->shader_ids;
@@ -242,11 +231,30 @@ aur_status check_params(const aur_render_params* p) {
     return AUR_OK;
 }
 
-int stack_cap(const aur_scene* sc) { return (int)sc->nmh->levels + 1; }
-
 }  // namespace aur
 
 using namespace aur;
+
+namespace {
+
+// Calls f with the scene's kernel variant: specular materials (the integrator
+// with the ray stack), the MIS estimator, few triangles.
+template <typename F>
+void launch_variant(const aur_scene* scene, bool mis, F f) {
+    auto pick = [&](auto spec, auto m) {
+        if (scene->nmh->count <= kTinyTris) f(spec, m, std::true_type{});
+        else f(spec, m, std::false_type{});
+    };
+    if (scene->has_specular) {
+        if (mis) pick(std::true_type{}, std::true_type{});
+        else pick(std::true_type{}, std::false_type{});
+    } else {
+        if (mis) pick(std::false_type{}, std::true_type{});
+        else pick(std::false_type{}, std::false_type{});
+    }
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -274,28 +282,15 @@ aur_status aur_render(aur_ctx* ctx, const aur_scene* scene, const aur_camera* ca
     float4* colors = nullptr;
     AUR_CHECK(::aur::dev_malloc_async(&colors, P * batch * sizeof(float4), ctx->stream) == cudaSuccess, AUR_ERR_OOM,
               "aur_render: out of device memory");
-    const int cap = stack_cap(scene);
-    const size_t smem = (size_t)2 * cap * kRenderThreads * sizeof(uint32_t);
     const SceneView sv = scene_view(scene);
     const float weight = 1.0f / (float)p.spp;
     for (uint32_t s = s0; s < s1; s += batch) {
         const uint32_t nb = std::min(batch, s1 - s);
         const dim3 grid(cdiv(P * nb, kRenderThreads));
-        if (scene->has_specular) {
-            if (mis)
-                k_render_samples<true, true><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, *camera, p, s, nb,
-                                                                                      colors, ctx->d_flags, cap);
-            else
-                k_render_samples<true, false><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, *camera, p, s, nb,
-                                                                                       colors, ctx->d_flags, cap);
-        } else {
-            if (mis)
-                k_render_samples<false, true><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, *camera, p, s, nb,
-                                                                                       colors, ctx->d_flags, cap);
-            else
-                k_render_samples<false, false><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, *camera, p, s, nb,
-                                                                                        colors, ctx->d_flags, cap);
-        }
+        launch_variant(scene, mis, [&](auto spec, auto m, auto tiny) {
+            k_render_samples<spec.value, m.value, tiny.value><<<grid, kRenderThreads, 0, ctx->stream>>>(
+                sv, *camera, p, s, nb, colors, ctx->d_flags);
+        });
         k_accumulate<<<cdiv(P, 256), 256, 0, ctx->stream>>>(colors, (uint32_t)P, nb, weight, (float4*)accum);
     }
     cudaFreeAsync(colors, ctx->stream);
@@ -335,28 +330,15 @@ aur_status aur_raytrace_monte_carlo(aur_ctx* ctx, const aur_scene* scene, const 
         st = build_mis_table(ctx, scene);
         if (st != AUR_OK) return st;
     }
-    const int cap = stack_cap(scene);
-    const size_t smem = (size_t)2 * cap * kRenderThreads * sizeof(uint32_t);
     const dim3 grid(cdiv(num_rays, kRenderThreads));
     const SceneView sv = scene_view(scene);
     const aur_render_params& p = *params;
     aur_path_ray* r = rays;
     aur_hitpoint* h = hits;
-    if (scene->has_specular) {
-        if (mis)
-            k_raytrace_mc<true, true><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, p, sample_id, offset, num_rays,
-                                                                                  r, h, ctx->d_flags, cap);
-        else
-            k_raytrace_mc<true, false><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, p, sample_id, offset,
-                                                                                   num_rays, r, h, ctx->d_flags, cap);
-    } else {
-        if (mis)
-            k_raytrace_mc<false, true><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, p, sample_id, offset,
-                                                                                   num_rays, r, h, ctx->d_flags, cap);
-        else
-            k_raytrace_mc<false, false><<<grid, kRenderThreads, smem, ctx->stream>>>(sv, p, sample_id, offset,
-                                                                                    num_rays, r, h, ctx->d_flags, cap);
-    }
+    launch_variant(scene, mis, [&](auto spec, auto m, auto tiny) {
+        k_raytrace_mc<spec.value, m.value, tiny.value><<<grid, kRenderThreads, 0, ctx->stream>>>(
+            sv, p, sample_id, offset, num_rays, r, h, ctx->d_flags);
+    });
     AUR_CUDA(cudaGetLastError());
     return AUR_OK;
 }

