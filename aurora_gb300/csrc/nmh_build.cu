@@ -395,34 +395,48 @@ __device__ __forceinline__ unsigned long long st_word(unsigned long long state, 
     return state | ((d & 0x7FFFFFFFull) << 31) | (l & 0x7FFFFFFFull);
 }
 
-// One thread: exclusive (D, L) prefix of `tile` given its own counts.
+__device__ __forceinline__ unsigned long long status_read(const unsigned long long* p) {
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    return w;
+}
+
+// One warp (all 32 lanes): exclusive (D, L) prefix of `tile` given its own
+// counts. The lanes read the 32 nearest predecessors at once: a word at a time
+// the walk over up to 244 tiles was most of these kernels' time (1M triangles:
+// split 22 us a level).
 __device__ uint2 tile_lookback(unsigned long long* status, uint32_t tile, uint32_t cd, uint32_t cl,
                                uint32_t* err, uint32_t test) {
-    if (tile == 0) {
-        atomicExch(status, st_word(kStPrefix, cd, cl));
-        return make_uint2(0u, 0u);
-    }
-    atomicExch(status + tile, st_word(kStTile, cd, cl));
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) atomicExch(status + tile, st_word(tile == 0 ? kStPrefix : kStTile, cd, cl));
+    if (tile == 0) return make_uint2(0u, 0u);
     uint64_t ed = 0, el = 0;
     uint32_t spins = 0;
     const uint32_t limit = test ? test : kLookbackSpins;
-    for (int64_t p = (int64_t)tile - 1; p >= 0;) {
-        const unsigned long long w = atomicAdd(status + p, 0ull);   // coherent read
-        const unsigned long long state = test ? 0ull : w >> 62;
-        if (state == 0) {
+    for (int64_t p = (int64_t)tile - 1 - lane;;) {
+        // before the first tile: an empty prefix
+        const unsigned long long w = p >= 0 ? status_read(status + p) : kStPrefix;
+        const uint32_t state = test ? 0u : (uint32_t)(w >> 62);
+        const uint32_t prefix = __ballot_sync(0xffffffffu, state == 2u);
+        const uint32_t unready = __ballot_sync(0xffffffffu, state == 0u);
+        const uint32_t upto = prefix ? (uint32_t)__ffs(prefix) : 32u;      // lanes [0, upto) count
+        if (unready & (upto == 32u ? 0xffffffffu : (1u << upto) - 1u)) {
             if (++spins > limit) {
-                atomicOr(err, kErrLookback);
+                if (lane == 0) atomicOr(err, kErrLookback);
                 break;
             }
             __nanosleep(32);
             continue;
         }
-        ed += (w >> 31) & 0x7FFFFFFFull;
-        el += w & 0x7FFFFFFFull;
-        if (state == 2) break;
-        --p;
+        uint64_t d = (uint32_t)lane < upto ? (w >> 31) & 0x7FFFFFFFull : 0ull;
+        uint64_t l = (uint32_t)lane < upto ? w & 0x7FFFFFFFull : 0ull;
+        // counts are below 2^30 each: two 32-bit sums
+        ed += __reduce_add_sync(0xffffffffu, (uint32_t)d);
+        el += __reduce_add_sync(0xffffffffu, (uint32_t)l);
+        if (prefix) break;
+        p -= 32;
     }
-    atomicExch(status + tile, st_word(kStPrefix, ed + cd, el + cl));
+    if (lane == 0) atomicExch(status + tile, st_word(kStPrefix, ed + cd, el + cl));
     return make_uint2((uint32_t)ed, (uint32_t)el);
 }
 
@@ -470,10 +484,11 @@ __device__ __forceinline__ void tile_scan(const uint32_t* __restrict__ list, uin
     }
     if (lane == 0) { s_d[warp] = cd; s_l[warp] = cl; }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
         uint32_t td = 0, tl = 0;
         for (int w = 0; w < kThreads / 32; ++w) { td += s_d[w]; tl += s_l[w]; }
-        s_pre = tile_lookback(status, s.tile, td, tl, err, test);
+        const uint2 pre = tile_lookback(status, s.tile, td, tl, err, test);
+        if (lane == 0) s_pre = pre;
     }
     __syncthreads();
     uint32_t od = s_pre.x, ol = s_pre.y;
@@ -703,21 +718,45 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_finish(const uint32_t* 
         __syncthreads();
         // select: pair[0] = first of the segment on axis a, pair[1] = arg-max
         // of (max-key, lowest prim id) over the rest (k_select)
-        for (uint32_t j = t; j < m; j += kLocalThreads) {
-            const uint16_t lid = s.list[cur][a][j];
-            const uint32_t r = lid < len ? s.node[lid] : kLocalDone;
-            if (r >= nd) {   // consistency check: every listed triangle belongs to a node of this depth
-                atomicOr(err, 4u);
-                continue;
+        // (runs of one node in a thread's four positions, then across the warp,
+        // before the atomic: at the subtree's first levels all entries belong to
+        // a few nodes)
+        {
+            uint32_t run = kLocalDone;
+            unsigned long long run_key = 0ull;
+#pragma unroll
+            for (int i = 0; i < kLocalPer; ++i) {
+                const uint32_t j = (uint32_t)t * kLocalPer + i;
+                if (j >= m) continue;
+                const uint16_t lid = s.list[cur][a][j];
+                const uint32_t r = lid < len ? s.node[lid] : kLocalDone;
+                if (r >= nd) {   // consistency check: every listed triangle belongs to a node of this depth
+                    atomicOr(err, 4u);
+                    continue;
+                }
+                unsigned long long key = 0ull;
+                if (j == s.off[r]) {
+                    s.p0[r] = lid;
+                } else {
+                    const uint32_t gp = s.pid[lid];
+                    key = ((unsigned long long)orderable(mx[a * S + gp]) << 32) | (unsigned long long)(0xFFFFFFFFu - gp);
+                }
+                if (r != run) {
+                    if (run != kLocalDone) atomicMax(&s.best[run], run_key);
+                    run = r;
+                    run_key = key;
+                } else if (key > run_key) {
+                    run_key = key;
+                }
             }
-            if (j == s.off[r]) {
-                s.p0[r] = lid;
-            } else {
-                const uint32_t gp = s.pid[lid];
-                const unsigned long long key =
-                    ((unsigned long long)orderable(mx[a * S + gp]) << 32) | (unsigned long long)(0xFFFFFFFFu - gp);
-                atomicMax(&s.best[r], key);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t on = __shfl_down_sync(0xffffffffu, run, o);
+                const unsigned long long ok = __shfl_down_sync(0xffffffffu, run_key, o);
+                if ((t & 31) + o < 32 && on == run && ok > run_key) run_key = ok;
             }
+            const uint32_t prev = __shfl_up_sync(0xffffffffu, run, 1);
+            if (run != kLocalDone && run_key != 0ull && ((t & 31) == 0 || prev != run)) atomicMax(&s.best[run], run_key);
         }
         __syncthreads();
         // emit (k_emit_pairs)
@@ -838,64 +877,6 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_finish(const uint32_t* 
     }
 }
 
-// Orders each pair by (min-key on the last level's axis, prim id).
-__global__ void k_pair_order(uint32_t n, const uint32_t* __restrict__ heap, const float* __restrict__ mn_last,
-                             uint32_t* __restrict__ perm, const uint32_t* err) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || build_aborted(err)) return;
-    uint32_t p = heap[2 * k], q = heap[2 * k + 1];
-    const float kp = mn_last[p], kq = mn_last[q];
-    if (kq < kp || (kq == kp && q < p)) { const uint32_t t = p; p = q; q = t; }
-    perm[2 * k] = p;
-    perm[2 * k + 1] = q;
-}
-
-// applyIndices (rebuilder.cu:217-245) for the vertices, plus the traversal
-// record of each node: slab of the pair on the node's axis
-// (intersect.cuh:106-111) and both triangles as (v1, e1, e2). The bounding
-// box of the pair goes to box[6k..6k+5] (lo.xyz, hi.xyz) for k_node_boxes.
-__global__ void k_emit_nodes(const float* __restrict__ V, uint32_t count_in, const uint32_t* __restrict__ perm,
-                             uint32_t n, float* __restrict__ verts, float4* __restrict__ recs,
-                             float* __restrict__ box, const uint32_t* err) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || build_aborted(err)) return;
-    const int a = (int)(level_of(k) % 3u);
-    float c[2][9];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const uint32_t pid = perm[2 * k + t];
-        const uint32_t src = pid < count_in ? pid : count_in - 1;
-        const float* v = V + (size_t)src * 9;
-        float* o = verts + (size_t)(2 * k + t) * 9;
-#pragma unroll
-        for (int q = 0; q < 9; ++q) { c[t][q] = v[q]; o[q] = c[t][q]; }
-    }
-    float blo[3], bhi[3];
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        blo[ax] = fminf(fminf(fminf(c[0][3 * ax], c[0][3 * ax + 1]), c[0][3 * ax + 2]),
-                        fminf(fminf(c[1][3 * ax], c[1][3 * ax + 1]), c[1][3 * ax + 2]));
-        bhi[ax] = fmaxf(fmaxf(fmaxf(c[0][3 * ax], c[0][3 * ax + 1]), c[0][3 * ax + 2]),
-                        fmaxf(fmaxf(c[1][3 * ax], c[1][3 * ax + 1]), c[1][3 * ax + 2]));
-        box[6 * (size_t)k + ax] = blo[ax];
-        box[6 * (size_t)k + 3 + ax] = bhi[ax];
-    }
-    float r[20];
-    r[0] = a == 0 ? blo[0] : (a == 1 ? blo[1] : blo[2]);
-    r[1] = a == 0 ? bhi[0] : (a == 1 ? bhi[1] : bhi[2]);
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        // layout [x1 x2 x3 y1 y2 y3 z1 z2 z3]: v1 = (c0, c3, c6), v2 = (c1, c4, c7), v3 = (c2, c5, c8)
-        float* o = r + 2 + 9 * t;
-        o[0] = c[t][0]; o[1] = c[t][3]; o[2] = c[t][6];
-        o[3] = c[t][1] - c[t][0]; o[4] = c[t][4] - c[t][3]; o[5] = c[t][7] - c[t][6];
-        o[6] = c[t][2] - c[t][0]; o[7] = c[t][5] - c[t][3]; o[8] = c[t][8] - c[t][6];
-    }
-    float4* rec = recs + (size_t)k * kRecStride;
-#pragma unroll
-    for (int q = 0; q < 5; ++q) rec[q] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-}
-
 // Box padding: relative 1e-5 of the coordinates' magnitude, far above the
 // rounding of the triangle test and of the box test.
 __device__ __forceinline__ void pad_interval(float lo, float hi, float& plo, float& phi) {
@@ -904,46 +885,132 @@ __device__ __forceinline__ void pad_interval(float lo, float hi, float& plo, flo
     phi = hi + p;
 }
 
-// Nodes [L0, L1) (kUnion: one heap level, bottom-up): with kUnion, sbox[k]
-// becomes the bounding box of node k's subtree (its pair's box pbox[k] and
-// its children's subtree boxes, computed one launch earlier); in both forms
-// the padded subtree boxes of the children go into record words 5..7 of
-// node k (an empty box where a child does not exist).
-template <bool kUnion>
-__global__ void k_node_boxes(uint32_t L0, uint32_t L1, uint32_t n, const float* __restrict__ pbox,
-                             float* __restrict__ box, float4* __restrict__ recs, const uint32_t* err) {
-    const uint32_t k = L0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= L1 || build_aborted(err)) return;
-    float b[6];
-    if (kUnion) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) b[q] = pbox[6 * (size_t)k + q];
-    }
-    float cb[2][6];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const uint32_t c = 2 * k + 1 + j;
-        if (c < n) {
+// Subtree boxes (box[6k..6k+5]: lo.xyz, hi.xyz) of the nodes of heap levels
+// [lv0, lv1), bottom-up: the bounds of a node's pair (k_bounds' min / max) and
+// its children's subtree boxes. One block walks all the levels of up to
+// kBoxThreads nodes in one launch; larger ones take a launch each, of as many
+// blocks.
+constexpr uint32_t kBoxThreads = 1024;
+
+__global__ void __launch_bounds__(kBoxThreads) k_upper_boxes(uint32_t lv0, uint32_t lv1, uint32_t n, size_t S,
+                                                             const uint32_t* __restrict__ heap,
+                                                             const float* __restrict__ mn, const float* __restrict__ mx,
+                                                             float* box, const uint32_t* err) {
+    if (build_aborted(err)) return;       // whole blocks: the word does not change during this launch
+    for (uint32_t lv = lv1; lv-- > lv0;) {
+        const uint32_t L0 = (1u << lv) - 1u, L1 = min((2u << lv) - 1u, n);
+        const uint32_t k = L0 + blockIdx.x * kBoxThreads + threadIdx.x;
+        if (k < L1) {
+            const uint32_t p = heap[2 * k], q = heap[2 * k + 1];
+            float b[6];
 #pragma unroll
             for (int ax = 0; ax < 3; ++ax) {
-                const float lo = box[6 * (size_t)c + ax], hi = box[6 * (size_t)c + 3 + ax];
-                b[ax] = fminf(b[ax], lo);
-                b[3 + ax] = fmaxf(b[3 + ax], hi);
-                pad_interval(lo, hi, cb[j][ax], cb[j][3 + ax]);
+                b[ax] = fminf(mn[ax * S + p], mn[ax * S + q]);
+                b[3 + ax] = fmaxf(mx[ax * S + p], mx[ax * S + q]);
             }
-        } else {
 #pragma unroll
-            for (int ax = 0; ax < 3; ++ax) { cb[j][ax] = 1.0f; cb[j][3 + ax] = -1.0f; }
+            for (int j = 0; j < 2; ++j) {
+                const uint32_t c = 2 * k + 1 + j;
+                if (c < n) {
+#pragma unroll
+                    for (int ax = 0; ax < 3; ++ax) {
+                        b[ax] = fminf(b[ax], box[6 * (size_t)c + ax]);
+                        b[3 + ax] = fmaxf(b[3 + ax], box[6 * (size_t)c + 3 + ax]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q6 = 0; q6 < 6; ++q6) box[6 * (size_t)k + q6] = b[q6];
+        }
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ void st_sector(float4* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
+// The NMH's arrays from the placed pairs, kEmitNodes nodes per block: each
+// pair ordered by (min-key on the last level's axis, prim id), the vertices in
+// that order (applyIndices, rebuilder.cu:217-245) and the traversal record of
+// each node: slab of the pair on the node's axis (intersect.cuh:106-111), both
+// triangles as (v1, e1, e2), and the padded subtree boxes of the children (an
+// empty box where a child does not exist). The vertices go through shared
+// memory, so that the gather and the copy out walk consecutive words; a record
+// is written as four whole 32-byte sectors. (1M triangles: 45 us; pair order,
+// vertices with half-written records, and the boxes in ten further launches
+// took 138 us.)
+constexpr uint32_t kEmitNodes = 128;
+
+__global__ void __launch_bounds__(kEmitNodes) k_emit_nodes(const float* __restrict__ V, uint32_t count_in, uint32_t n,
+                                                           const uint32_t* __restrict__ heap,
+                                                           const float* __restrict__ mn_last,
+                                                           const float* __restrict__ box, uint32_t* __restrict__ perm,
+                                                           float* __restrict__ verts, float4* __restrict__ recs,
+                                                           const uint32_t* err) {
+    __shared__ uint32_t s_src[2 * kEmitNodes];
+    __shared__ float s_v[18 * kEmitNodes];
+    if (build_aborted(err)) return;       // whole blocks: the word does not change during this launch
+    const uint32_t k0 = blockIdx.x * kEmitNodes, t = threadIdx.x, k = k0 + t;
+    const uint32_t m = min(kEmitNodes, n - k0);      // nodes of this block
+    if (k < n) {
+        uint32_t p = heap[2 * (size_t)k], q = heap[2 * (size_t)k + 1];
+        const float kp = mn_last[p], kq = mn_last[q];
+        if (kq < kp || (kq == kp && q < p)) { const uint32_t x = p; p = q; q = x; }
+        perm[2 * (size_t)k] = p;
+        perm[2 * (size_t)k + 1] = q;
+        s_src[2 * t] = p < count_in ? p : count_in - 1;
+        s_src[2 * t + 1] = q < count_in ? q : count_in - 1;
+    }
+    __syncthreads();
+    for (uint32_t j = t; j < 18u * m; j += kEmitNodes) s_v[j] = V[(size_t)s_src[j / 9u] * 9 + j % 9u];
+    __syncthreads();
+    float* out = verts + (size_t)k0 * 18;
+    for (uint32_t j = t; j < 18u * m; j += kEmitNodes) out[j] = s_v[j];
+    if (k >= n) return;
+    const int a = (int)(level_of(k) % 3u);
+    float c[2][9];
+#pragma unroll
+    for (int q = 0; q < 18; ++q) c[q / 9][q % 9] = s_v[18 * t + q];
+    float r[32];
+    {
+        float lo[3], hi[3];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            lo[ax] = fminf(fminf(fminf(c[0][3 * ax], c[0][3 * ax + 1]), c[0][3 * ax + 2]),
+                           fminf(fminf(c[1][3 * ax], c[1][3 * ax + 1]), c[1][3 * ax + 2]));
+            hi[ax] = fmaxf(fmaxf(fmaxf(c[0][3 * ax], c[0][3 * ax + 1]), c[0][3 * ax + 2]),
+                           fmaxf(fmaxf(c[1][3 * ax], c[1][3 * ax + 1]), c[1][3 * ax + 2]));
+        }
+        r[0] = a == 0 ? lo[0] : (a == 1 ? lo[1] : lo[2]);
+        r[1] = a == 0 ? hi[0] : (a == 1 ? hi[1] : hi[2]);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        // layout [x1 x2 x3 y1 y2 y3 z1 z2 z3]: v1 = (c0, c3, c6), v2 = (c1, c4, c7), v3 = (c2, c5, c8)
+        float* o = r + 2 + 9 * q;
+        o[0] = c[q][0]; o[1] = c[q][3]; o[2] = c[q][6];
+        o[3] = c[q][1] - c[q][0]; o[4] = c[q][4] - c[q][3]; o[5] = c[q][7] - c[q][6];
+        o[6] = c[q][2] - c[q][0]; o[7] = c[q][5] - c[q][3]; o[8] = c[q][8] - c[q][6];
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const uint32_t ch = 2 * k + 1 + j;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            r[20 + 6 * j + ax] = 1.0f;
+            r[23 + 6 * j + ax] = -1.0f;
+            if (ch < n)
+                pad_interval(box[6 * (size_t)ch + ax], box[6 * (size_t)ch + 3 + ax], r[20 + 6 * j + ax], r[23 + 6 * j + ax]);
         }
     }
-    if (kUnion) {
+    float4* rec = recs + (size_t)k * kRecStride;
 #pragma unroll
-        for (int q = 0; q < 6; ++q) box[6 * (size_t)k + q] = b[q];
-    }
-    float4* rec = recs + (size_t)k * kRecStride + 5;
-    rec[0] = make_float4(cb[0][0], cb[0][1], cb[0][2], cb[0][3]);
-    rec[1] = make_float4(cb[0][4], cb[0][5], cb[1][0], cb[1][1]);
-    rec[2] = make_float4(cb[1][2], cb[1][3], cb[1][4], cb[1][5]);
+    for (int q = 0; q < 4; ++q)
+        st_sector(rec + 2 * q, make_float4(r[8 * q], r[8 * q + 1], r[8 * q + 2], r[8 * q + 3]),
+                  make_float4(r[8 * q + 4], r[8 * q + 5], r[8 * q + 6], r[8 * q + 7]));
 }
 
 // One thread per treelet writes its record (wide_record) from the NMH-ordered
@@ -967,6 +1034,14 @@ uint32_t log2i(uint32_t x) {
 // Look-back scratch: per list (the split list and the two partitioned ones)
 // one status word per tile, then the three tile counters.
 constexpr size_t lookback_bytes(size_t ntiles) { return 3 * ntiles * sizeof(unsigned long long) + 16; }
+
+// No fewer than the levels that run over the whole soup (local_level): the
+// segments of level lv hold at most N / 2^lv triangles.
+constexpr size_t max_global_levels(size_t N) {
+    size_t lv = 0;
+    while ((N >> lv) > kLocalMax) ++lv;
+    return lv + 1;
+}
 
 // ------------------------------------------------------------ launch sequence
 //
@@ -1102,13 +1177,12 @@ private:
 };
 
 // One level's split of the next axis' list and partition of the other two,
-// each a single pass with look-back tile prefixes; the status words and
-// tile counters are cleared first.
+// each a single pass with look-back tile prefixes; lb: this level's status
+// words and tile counters, cleared with the build's other zeroed scratch.
 void split_and_partition(Seq& q, const ListSet& sb, const ListSet& sac, uint32_t M, uint32_t mt, uint32_t ntiles,
                          uint32_t* node_of, const uint32_t* ns, const uint32_t* nl, const uint32_t* nlb, uint32_t L0,
                          uint32_t m_next, unsigned long long* lb, uint32_t* err, uint32_t test) {
     uint32_t* counters = reinterpret_cast<uint32_t*>(lb + 3 * (size_t)ntiles);
-    q.memset(lb, lookback_bytes(ntiles));
     q.launch(k_split_next, dim3(mt), dim3(kThreads), 0, sb, M, node_of, ns, nl, L0, lb, counters, err, test);
     q.launch(k_partition, dim3(mt, 2), dim3(kThreads), 0, sac, M, node_of, ns, nl, nlb, L0, lb + ntiles, ntiles,
              counters + 1, m_next, err, test);
@@ -1131,30 +1205,12 @@ void finish_local(Seq& q, const uint32_t* list, size_t S, const float* mn, const
              nstart, 2 * n, node_of, heap, sbox, err);
 }
 
-// Node records: pairs and slabs, then the children's subtree boxes. The
-// subtree boxes of levels >= lv0 are in sbox already (k_local_finish); the
-// levels above are unions, level by level from the bottom, of the pair boxes
-// (pbox, written by k_emit_nodes) and the children's subtree boxes.
-// pbox and sbox: 6 floats per node of scratch each.
-void emit_records(Seq& q, const float* V, uint32_t count, const uint32_t* perm, uint32_t n, uint32_t lv0,
-                  float* verts, float4* recs, float* pbox, float* sbox, const uint32_t* err) {
-    q.launch(k_emit_nodes, dim3(cdiv(n, 128)), dim3(128), 0, V, count, perm, n, verts, recs, pbox, err);
-    const uint32_t Lb = (1u << lv0) - 1u;   // first node of level lv0
-    if (Lb < n)
-        q.launch(k_node_boxes<false>, dim3(cdiv(n - Lb, 256)), dim3(256), 0, Lb, n, n, pbox, sbox, recs, err);
-    for (int lv = (int)lv0 - 1; lv >= 0; --lv) {
-        const uint32_t L0 = (1u << lv) - 1u;
-        const uint32_t L1 = ((2u << lv) - 1u) < n ? ((2u << lv) - 1u) : n;
-        q.launch(k_node_boxes<true>, dim3(cdiv(L1 - L0, 256)), dim3(256), 0, L0, L1, n, pbox, sbox, recs, err);
-    }
-}
-
 constexpr size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Byte offsets of the scratch regions of a build of N (even) triangles; the
 // per-axis arrays use a stride S that keeps every axis 256-byte aligned.
 struct ScratchLayout {
-    size_t S, flags, mn, mx, keys, vals, k2, v2, nodeof, heap, pair0, best, ns, nl, nlb, tiles, hist, tot, end;
+    size_t S, flags, mn, mx, keys, vals, k2, v2, zero, zero_end, nodeof, heap, pair0, best, ns, nl, nlb, tiles, hist, tot, end;
 };
 
 constexpr ScratchLayout scratch_layout(size_t N) {
@@ -1171,14 +1227,16 @@ constexpr ScratchLayout scratch_layout(size_t N) {
     L.vals = off; off += round256(3 * L.S * 4);
     L.k2 = off; off += round256(3 * L.S * 4);
     L.v2 = off; off += round256(3 * L.S * 4);
+    L.zero = off;                       // cleared before each build, up to zero_end
     L.nodeof = off; off += round256(N * 4);
+    L.best = off; off += round256(n * 8);
+    L.tiles = off; off += round256(max_global_levels(N) * lookback_bytes(ntiles));
+    L.zero_end = off;
     L.heap = off; off += round256(N * 4);
     L.pair0 = off; off += round256(n * 4);
-    L.best = off; off += round256(n * 8);
     L.ns = off; off += round256(n * 4);
     L.nl = off; off += round256(n * 4);
     L.nlb = off; off += round256(n * 4);
-    L.tiles = off; off += round256(lookback_bytes(ntiles));
     L.hist = off; off += round256(3 * 256 * nb * 4);
     L.tot = off; off += round256(3 * 256 * 4);
     L.end = off;
@@ -1197,6 +1255,20 @@ struct BuildArgs {
     uint4* wide = nullptr;     // treelet records (wide_count(levels)), or null: not built
     uint32_t lookback_test = 0;  // test hook: nonzero makes the look-back waits run out (see tile_lookback)
 };
+
+// The subtree boxes of the levels above lv0 (those of lv0 and below are in
+// sbox already, k_local_finish), then the NMH's arrays.
+void emit_records(Seq& q, const BuildArgs& b, uint32_t n, uint32_t levels, uint32_t lv0, size_t S, const uint32_t* heap,
+                  const float* mn, const float* mx, float* sbox) {
+    uint32_t lv = lv0;
+    for (; lv > 0 && (1u << (lv - 1)) > kBoxThreads; --lv)
+        q.launch(k_upper_boxes, dim3(cdiv(1u << (lv - 1), kBoxThreads)), dim3(kBoxThreads), 0, lv - 1, lv, n, S, heap, mn,
+                 mx, sbox, b.flags);
+    if (lv > 0)
+        q.launch(k_upper_boxes, dim3(1), dim3(kBoxThreads), 0, 0u, lv, n, S, heap, mn, mx, sbox, b.flags);
+    q.launch(k_emit_nodes, dim3(cdiv(n, kEmitNodes)), dim3(kEmitNodes), 0, b.V, b.count, n, heap,
+             mn + ((levels - 1) % 3) * S, (const float*)sbox, b.perm, b.verts, b.recs, b.flags);
+}
 
 // The whole build of a non-empty soup: bounds and keys, three radix sorts,
 // the global levels, the per-subtree finish, pair order and node records.
@@ -1226,8 +1298,7 @@ void enqueue_build(Seq& q, const BuildArgs& b) {
     const uint32_t nb = cdiv(N, kSortTile);
     const uint32_t ntiles = cdiv(N, kTile);
 
-    q.memset(node_of, (size_t)N * 4);
-    q.memset(best, (size_t)n * 8);
+    q.memset(base + L.zero, L.zero_end - L.zero);
     q.launch(k_bounds, dim3(cdiv(N, 256)), dim3(256), 0, b.V, N, S, b.count, mn, mx, keys, vals, b.flags);
     // three stable LSD radix sorts of (min-key, prim id); result in keys/vals
     for (int pass = 0; pass < 4; ++pass) {
@@ -1266,15 +1337,14 @@ void enqueue_build(Seq& q, const BuildArgs& b) {
         ListSet sac;
         sac.in[0] = listA + a * S; sac.out[0] = listB + a * S;
         sac.in[1] = listA + c * S; sac.out[1] = listB + c * S;
-        split_and_partition(q, sb, sac, M, mt, ntiles, node_of, ns, nl, nlb, L0, M - 2u * (L1 - L0), tiles, b.flags,
+        split_and_partition(q, sb, sac, M, mt, ntiles, node_of, ns, nl, nlb, L0, M - 2u * (L1 - L0),
+                            tiles + lv * (lookback_bytes(ntiles) / sizeof(unsigned long long)), b.flags,
                             b.lookback_test);
         uint32_t* t = listA; listA = listB; listB = t;
     }
     if (lv0 < levels) finish_local(q, listA, S, mn, mx, n, lv0, ns, node_of, heap, (float*)k2, b.flags);
-    const int al = (int)((levels - 1) % 3);
-    q.launch(k_pair_order, dim3(cdiv(n, 256)), dim3(256), 0, n, heap, mn + al * S, b.perm, b.flags);
-    // mx and k2 are free once the levels are placed: 3*S >= 6*n floats each for the boxes
-    emit_records(q, b.V, b.count, b.perm, n, lv0, b.verts, b.recs, mx, (float*)k2, b.flags);
+    // k2 is free once the levels are placed: 3*S >= 6*n floats for the boxes
+    emit_records(q, b, n, levels, lv0, S, heap, mn, mx, (float*)k2);
     if (b.wide) {
         const uint32_t treelets = (uint32_t)wide_count(levels);
         q.launch(k_wide_nodes, dim3(cdiv(treelets, 128)), dim3(128), 0, b.verts, (const float*)k2, n, levels, treelets,
