@@ -584,70 +584,54 @@ constexpr int kLocalThreads = 512;
 constexpr int kLocalPer = (int)kLocalMax / kLocalThreads;   // elements per thread in block scans
 constexpr uint16_t kLocalDone = 0xFFFFu;
 
-// 53.6 KB: four blocks fit an SM, so the 512 subtrees of a 1M-triangle
+// 54.1 KB: four blocks fit an SM, so the 512 subtrees of a 1M-triangle
 // build run as one wave on 152 SMs.
 struct LocalSmem {
     uint16_t list[2][3][kLocalMax];       // local ids, double-buffered, per axis
     uint16_t node[kLocalMax];             // local node index at the current depth, kLocalDone once paired
     uint8_t right[kLocalMax];             // 1: goes to the right child at the next depth
-    union {                               // select / emit use best, split / partition the scans
-        struct {
-            uint16_t pre0[kLocalMax];     // block-scan outputs (exclusive prefix counts)
-            uint16_t pre1[kLocalMax];
-        };
-        unsigned long long best[kLocalMax / 2];
-    };
+    unsigned long long best[kLocalMax / 2];
     uint32_t pid[kLocalMax];              // global prim id of each local id
     uint16_t off[kLocalMax / 2 + 1];      // segment offsets of the depth's nodes (+ end)
     uint16_t numl[kLocalMax / 2];         // triangles going to the left child
+    uint16_t lbase[kLocalMax / 2];        // and those of the nodes before
     uint16_t p0[kLocalMax / 2];           // pair[0] (local id) per node
-    uint32_t warp_tot[kLocalThreads / 32][2];
+    uint2 warp_tot[kLocalThreads / 32];
 };
 
-// Exclusive prefix counts of two flags over positions [0, m) (each thread a
-// contiguous chunk of kLocalPer), written to out0 and (if not null) out1;
-// returns the totals.
-template <typename F>
-__device__ __forceinline__ void local_scan2(LocalSmem& s, uint32_t m, F flags, uint16_t* out0, uint16_t* out1,
-                                            uint32_t& tot0, uint32_t& tot1) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t b = (uint32_t)t * kLocalPer;
-    uint32_t f0[kLocalPer], f1[kLocalPer];
-    uint32_t c0 = 0, c1 = 0;
-#pragma unroll
-    for (int i = 0; i < kLocalPer; ++i) {
-        f0[i] = f1[i] = 0;
-        if (b + i < m) flags(b + i, f0[i], f1[i]);
-        c0 += f0[i];
-        c1 += f1[i];
-    }
-    uint32_t x0 = c0, x1 = c1;
+// Exclusive block-wide prefix of (x, y), one pair per thread: two 16-bit
+// counts each.
+__device__ __forceinline__ uint2 local_scan(LocalSmem& s, uint2 v) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint2 x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y0 = __shfl_up_sync(0xffffffffu, x0, o), y1 = __shfl_up_sync(0xffffffffu, x1, o);
-        if (lane >= o) { x0 += y0; x1 += y1; }
+        const uint32_t a = __shfl_up_sync(0xffffffffu, x.x, o), b = __shfl_up_sync(0xffffffffu, x.y, o);
+        if (lane >= o) { x.x += a; x.y += b; }
     }
-    if (lane == 31) { s.warp_tot[warp][0] = x0; s.warp_tot[warp][1] = x1; }
+    if (lane == 31) s.warp_tot[warp] = x;
     __syncthreads();
-    uint32_t w0 = 0, w1 = 0, a0 = 0, a1 = 0;
-    for (int w = 0; w < kLocalThreads / 32; ++w) {
-        if (w < warp) { w0 += s.warp_tot[w][0]; w1 += s.warp_tot[w][1]; }
-        a0 += s.warp_tot[w][0];
-        a1 += s.warp_tot[w][1];
-    }
-    uint32_t r0 = w0 + x0 - c0, r1 = w1 + x1 - c1;
+    const uint2 w = lane < warp ? s.warp_tot[lane] : make_uint2(0u, 0u);     // the warps before (16 in all)
+    const uint32_t wx = __reduce_add_sync(0xffffffffu, w.x), wy = __reduce_add_sync(0xffffffffu, w.y);
+    return make_uint2(wx + x.x - v.x, wy + x.y - v.y);
+}
+
+// A thread's kLocalPer consecutive list entries.
+struct LocalItems {
+    uint32_t lid[kLocalPer], node[kLocalPer];   // node kLocalDone: past the end, or retired
+    bool in[kLocalPer];
+};
+__device__ __forceinline__ LocalItems local_items(const LocalSmem& s, const uint16_t* list, uint32_t m, uint32_t len) {
+    LocalItems it;
+    const uint32_t b = threadIdx.x * kLocalPer;
+    const ushort4 v = *reinterpret_cast<const ushort4*>(list + b);
+    it.lid[0] = v.x; it.lid[1] = v.y; it.lid[2] = v.z; it.lid[3] = v.w;
 #pragma unroll
     for (int i = 0; i < kLocalPer; ++i) {
-        if (b + i < m) {
-            out0[b + i] = (uint16_t)r0;
-            if (out1) out1[b + i] = (uint16_t)r1;
-        }
-        r0 += f0[i];
-        r1 += f1[i];
+        it.in[i] = b + i < m;
+        it.node[i] = it.in[i] && it.lid[i] < len ? s.node[it.lid[i]] : kLocalDone;
     }
-    tot0 = a0;
-    tot1 = a1;
-    __syncthreads();
+    return it;
 }
 
 // Finishes the subtree of node L0 + blockIdx.x (levels lv0 .. levels-1).
@@ -658,6 +642,8 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_finish(const uint32_t* 
                                                                  const float* __restrict__ mx, uint32_t n,
                                                                  uint32_t lv0, uint32_t L0,
                                                                  const uint32_t* __restrict__ nstart,
+                                                                 const uint32_t* __restrict__ nnuml,
+                                                                 const uint32_t* __restrict__ nlbase,
                                                                  uint32_t npids, uint32_t* __restrict__ lid_of,
                                                                  uint32_t* __restrict__ heap,
                                                                  float* __restrict__ sbox,
@@ -698,47 +684,42 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_finish(const uint32_t* 
         const uint64_t avail = (uint64_t)n - G0;
         const uint32_t nd = (uint32_t)((1ull << d) < avail ? (1ull << d) : avail);
         const uint32_t a = lv % 3u, b = (lv + 1) % 3u, c = (lv + 2) % 3u;
-        // node table of this depth: segment lengths and left sizes, offsets by a scan
+        // the depth's part of the node table (k_node_table), relative to this block's first node
         {
-            uint32_t tot0, tot1;
-            local_scan2(
-                s, nd,
-                [&](uint32_t r, uint32_t& f0, uint32_t& f1) {
-                    const uint64_t g = G0 + r;
-                    f0 = (uint32_t)(2 * subtree_nodes(g, n));
-                    f1 = 0;
-                    s.numl[r] = (uint16_t)((2 * g + 1 < n) ? 2 * subtree_nodes(2 * g + 1, n) : 0);
-                },
-                s.off, nullptr, tot0, tot1);
-            if (t == 0) s.off[nd] = (uint16_t)tot0;
-            __syncthreads();
+            const uint32_t o0 = nstart[G0], l0 = nlbase[G0];
+            for (uint32_t r = t; r < nd; r += kLocalThreads) {
+                const uint32_t o = nstart[G0 + r] - o0;
+                s.off[r] = (uint16_t)o;
+                s.numl[r] = (uint16_t)nnuml[G0 + r];
+                s.lbase[r] = (uint16_t)(nlbase[G0 + r] - l0);
+                s.best[r] = 0ull;
+                if (r == nd - 1) s.off[nd] = (uint16_t)(o + 2 * subtree_nodes(G0 + r, n));
+            }
         }
-        const uint32_t m = s.off[nd];
-        for (uint32_t r = t; r < nd; r += kLocalThreads) s.best[r] = 0ull;   // shares storage with the scans
         __syncthreads();
+        const uint32_t m = s.off[nd];
         // select: pair[0] = first of the segment on axis a, pair[1] = arg-max
         // of (max-key, lowest prim id) over the rest (k_select)
         // (runs of one node in a thread's four positions, then across the warp,
         // before the atomic: at the subtree's first levels all entries belong to
         // a few nodes)
         {
+            const LocalItems it = local_items(s, s.list[cur][a], m, len);
             uint32_t run = kLocalDone;
             unsigned long long run_key = 0ull;
 #pragma unroll
             for (int i = 0; i < kLocalPer; ++i) {
-                const uint32_t j = (uint32_t)t * kLocalPer + i;
-                if (j >= m) continue;
-                const uint16_t lid = s.list[cur][a][j];
-                const uint32_t r = lid < len ? s.node[lid] : kLocalDone;
+                if (!it.in[i]) continue;
+                const uint32_t r = it.node[i];
                 if (r >= nd) {   // consistency check: every listed triangle belongs to a node of this depth
                     atomicOr(err, 4u);
                     continue;
                 }
                 unsigned long long key = 0ull;
-                if (j == s.off[r]) {
-                    s.p0[r] = lid;
+                if ((uint32_t)t * kLocalPer + i == s.off[r]) {
+                    s.p0[r] = (uint16_t)it.lid[i];
                 } else {
-                    const uint32_t gp = s.pid[lid];
+                    const uint32_t gp = s.pid[it.lid[i]];
                     key = ((unsigned long long)orderable(mx[a * S + gp]) << 32) | (unsigned long long)(0xFFFFFFFFu - gp);
                 }
                 if (r != run) {
@@ -778,63 +759,80 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_finish(const uint32_t* 
         if (2 * G0 + 1 >= n) break;   // no node below this depth
         const int nxt = cur ^ 1;
         // split the next axis' list: drop the pairs, rank within the node's
-        // remainder decides left / right (k_split_next)
+        // remainder decides left / right (k_split_next); 2 r entries are
+        // retired before node r's segment
         {
-            uint32_t td, tu;
-            local_scan2(
-                s, m,
-                [&](uint32_t j, uint32_t& f0, uint32_t& f1) {
-                    const uint16_t lid = s.list[cur][b][j];
-                    f0 = lid < len && s.node[lid] == kLocalDone;
-                    f1 = 0;
-                },
-                s.pre0, nullptr, td, tu);
-            for (uint32_t j = t; j < m; j += kLocalThreads) {
-                const uint16_t lid = s.list[cur][b][j];
-                const uint32_t r = lid < len ? s.node[lid] : kLocalDone;
-                if (r == kLocalDone) continue;
+            const LocalItems it = local_items(s, s.list[cur][b], m, len);
+            uint32_t c0 = 0;
+#pragma unroll
+            for (int i = 0; i < kLocalPer; ++i) c0 += it.in[i] && it.node[i] == kLocalDone;
+            uint32_t db = local_scan(s, make_uint2(c0, 0u)).x;
+#pragma unroll
+            for (int i = 0; i < kLocalPer; ++i) {
+                const uint32_t j = (uint32_t)t * kLocalPer + i, r = it.node[i];
+                if (r == kLocalDone) {
+                    db += it.in[i];
+                    continue;
+                }
                 if (r >= nd) {
                     atomicOr(err, 4u);
                     continue;
                 }
-                const uint32_t db = s.pre0[j];
                 const uint32_t rpos = (j - s.off[r]) - (db - 2u * r);
-                s.right[lid] = rpos < s.numl[r] ? 0 : 1;
-                s.list[nxt][b][j - db] = lid;
+                s.right[it.lid[i]] = rpos < s.numl[r] ? 0 : 1;
+                s.list[nxt][b][j - db] = (uint16_t)it.lid[i];
             }
             __syncthreads();
         }
         // stable partition of the other two lists into left then right child
-        // segments (k_partition)
-        for (int which = 0; which < 2; ++which) {
-            const uint32_t x = which == 0 ? a : c;
-            uint32_t td, tl;
-            local_scan2(
-                s, m,
-                [&](uint32_t j, uint32_t& f0, uint32_t& f1) {
-                    const uint16_t lid = s.list[cur][x][j];
-                    const bool done = lid >= len || s.node[lid] == kLocalDone;
-                    f0 = done;
-                    f1 = !done && !s.right[lid];
-                },
-                s.pre0, s.pre1, td, tl);
-            for (uint32_t j = t; j < m; j += kLocalThreads) {
-                const uint16_t lid = s.list[cur][x][j];
-                const uint32_t r = lid < len ? s.node[lid] : kLocalDone;
-                if (r == kLocalDone) continue;
-                if (r >= nd) {
-                    atomicOr(err, 4u);
-                    continue;
+        // segments (k_partition), both behind one scan
+        {
+            const LocalItems ia = local_items(s, s.list[cur][a], m, len), ic = local_items(s, s.list[cur][c], m, len);
+            uint2 cnt = make_uint2(0u, 0u);      // retired, and left << 16, of each list
+            uint32_t ra = 0, rc = 0;             // bit i: entry i goes right
+#pragma unroll
+            for (int i = 0; i < kLocalPer; ++i) {
+                if (ia.node[i] != kLocalDone) {
+                    const uint32_t x = s.right[ia.lid[i]];
+                    ra |= x << i;
+                    cnt.x += x ? 0u : 0x10000u;
+                } else {
+                    cnt.x += ia.in[i];
                 }
-                const uint32_t o = s.off[r];
-                const uint32_t base = o - 2u * r;                 // left child's segment at the next depth
-                const uint32_t lb = s.pre1[j] - s.pre1[o];        // left elements of this node before j
-                const uint32_t db = s.pre0[j] - s.pre0[o];        // retired elements of this node before j
-                uint32_t dst;
-                if (!s.right[lid]) dst = base + lb;
-                else dst = base + s.numl[r] + ((j - o) - lb - db);
-                if (dst < m - 2u * nd) s.list[nxt][x][dst] = lid;
-                else atomicOr(err, 4u);
+                if (ic.node[i] != kLocalDone) {
+                    const uint32_t x = s.right[ic.lid[i]];
+                    rc |= x << i;
+                    cnt.y += x ? 0u : 0x10000u;
+                } else {
+                    cnt.y += ic.in[i];
+                }
+            }
+            const uint2 pre = local_scan(s, cnt);
+#pragma unroll
+            for (int which = 0; which < 2; ++which) {
+                const LocalItems& it = which ? ic : ia;
+                const uint32_t right = which ? rc : ra;
+                uint32_t db = (which ? pre.y : pre.x) & 0xFFFFu, lb = (which ? pre.y : pre.x) >> 16;
+                uint16_t* out = s.list[nxt][which ? c : a];
+#pragma unroll
+                for (int i = 0; i < kLocalPer; ++i) {
+                    const uint32_t j = (uint32_t)t * kLocalPer + i, r = it.node[i];
+                    if (r == kLocalDone) {
+                        db += it.in[i];
+                        continue;
+                    }
+                    if (r >= nd) {
+                        atomicOr(err, 4u);
+                        continue;
+                    }
+                    const uint32_t o = s.off[r], base = o - 2u * r;   // left child's segment at the next depth
+                    const uint32_t nl = lb - s.lbase[r];              // left elements of this node before j
+                    const bool rt = (right >> i) & 1u;
+                    const uint32_t dst = rt ? base + s.numl[r] + ((j - o) - nl - (db - 2u * r)) : base + nl;
+                    lb += rt ? 0u : 1u;
+                    if (dst < m - 2u * nd) out[dst] = (uint16_t)it.lid[i];
+                    else atomicOr(err, 4u);
+                }
             }
             __syncthreads();
         }
@@ -1198,11 +1196,12 @@ uint32_t local_level(uint32_t n, uint32_t levels) {
 
 // The remaining levels lv0 .. levels-1, one block per node of level lv0.
 void finish_local(Seq& q, const uint32_t* list, size_t S, const float* mn, const float* mx, uint32_t n, uint32_t lv0,
-                  const uint32_t* nstart, uint32_t* node_of, uint32_t* heap, float* sbox, uint32_t* err) {
+                  const uint32_t* nstart, const uint32_t* nnuml, const uint32_t* nlbase, uint32_t* node_of, uint32_t* heap,
+                  float* sbox, uint32_t* err) {
     const uint32_t L0 = (1u << lv0) - 1u;
     const uint32_t L1 = ((2u << lv0) - 1u) < n ? ((2u << lv0) - 1u) : n;
     q.launch(k_local_finish, dim3(L1 - L0), dim3(kLocalThreads), sizeof(LocalSmem), list, S, mn, mx, n, lv0, L0,
-             nstart, 2 * n, node_of, heap, sbox, err);
+             nstart, nnuml, nlbase, 2 * n, node_of, heap, sbox, err);
 }
 
 constexpr size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -1342,7 +1341,7 @@ void enqueue_build(Seq& q, const BuildArgs& b) {
                             b.lookback_test);
         uint32_t* t = listA; listA = listB; listB = t;
     }
-    if (lv0 < levels) finish_local(q, listA, S, mn, mx, n, lv0, ns, node_of, heap, (float*)k2, b.flags);
+    if (lv0 < levels) finish_local(q, listA, S, mn, mx, n, lv0, ns, nl, nlb, node_of, heap, (float*)k2, b.flags);
     // k2 is free once the levels are placed: 3*S >= 6*n floats for the boxes
     emit_records(q, b, n, levels, lv0, S, heap, mn, mx, (float*)k2);
     if (b.wide) {
