@@ -48,7 +48,7 @@ struct TreeTrav {
 };
 struct TinyTrav {
     static constexpr bool kTiny = true;
-    const float4* tris;    // stage_tiny's triangles
+    const TinyStage* stage;
     uint32_t count;
 };
 
@@ -57,10 +57,9 @@ struct TinyTrav {
 template <bool kTiny>
 __device__ __forceinline__ auto make_trav(const SceneView& sc) {
     if constexpr (kTiny) {
-        __shared__ float4 s_tri[3 * kTinyTris];
-        stage_tiny(s_tri, sc.verts, sc.perm, 2u * sc.nodes);
-        __syncthreads();
-        return TinyTrav{s_tri, 2u * sc.nodes};
+        __shared__ __align__(16) TinyStage s_stage;
+        stage_tiny(s_stage, sc.verts, sc.perm, 2u * sc.nodes);
+        return TinyTrav{&s_stage, 2u * sc.nodes};
     } else {
         return TreeTrav{};
     }
@@ -81,7 +80,7 @@ __device__ __forceinline__ uint32_t closest_hit(const SceneView& sc, const Trav&
     if constexpr (Trav::kTiny) {
         r.pos = pos;
         r.dir = dir;
-        tiny_closest(trav.tris, trav.count, pos, dir, tmax, h);
+        tiny_closest(*trav.stage, trav.count, pos, dir, tmax, h);
     } else {
         WideState s;
         if (wide_begin(r, s, h, w, pos, dir, tmax))
@@ -101,7 +100,7 @@ __device__ __forceinline__ bool occluded(const SceneView& sc, const Trav& trav, 
     if constexpr (Trav::kTiny) {
         r.pos = pos;
         r.dir = dir;
-        h.best = tiny_any(trav.tris, trav.count, pos, dir, tmax);
+        h.best = tiny_any(*trav.stage, trav.count, pos, dir, tmax);
     } else {
         WideState s;
         if (wide_begin(r, s, h, w, pos, dir, tmax))

@@ -611,38 +611,147 @@ __device__ __forceinline__ void wide_warp(const WideView& w, WideQueue& q, bool 
 // one address, so no lane waits for another's path and no load waits for a
 // node. (1M rays, 100 triangles: 0.20 ms so, 0.20 ms over the treelets; 34:
 // 0.10 ms against 0.19 ms.)
+//
+// A filter goes first, two triangles at a time in packed multiply-adds. With
+// m = pos x dir, the three signs Moller-Trumbore decides by are
+//   det     = dir . (e2 x e1)
+//   u * det = e2 . m + dir . (v1 x e2)
+//   v * det = -e1 . m - dir . (v1 x e1)
+// and the constants are staged. Their rounding, and that of intersect_tri's
+// own terms, is below 1.3e-6 (|pos| + R) |dir| times the longer edge (R: the
+// vertices' largest distance from the origin; at most a dozen roundings of
+// 2^-24 each on terms no larger); a triangle is dropped when a sign is wrong
+// by more than three times that, so every triangle intersect_tri accepts is
+// kept. The few kept ones are then tested exactly. (256x256 box frame, 16
+// samples: 0.96 ms without the filter, 0.86 with it; 1M rays, 34 triangles:
+// 0.10 and 0.08 ms.)
 constexpr uint32_t kTinyTris = 64;
 
-#ifdef __CUDACC__
-// Stages `count` triangles as (v1, prim id), e1, e2: 3 * count float4. The
-// whole block calls it, and synchronizes before reading them.
-__device__ __forceinline__ void stage_tiny(float4* __restrict__ s_tri, const float* __restrict__ verts,
+struct TinyStage {
+    float4 tri[3 * kTinyTris];          // (v1, prim id), e1, e2
+    float2 pre[kTinyTris / 2][16];      // of two triangles: e2 x e1, e2, v1 x e2, -e1, -(v1 x e1), longer edge
+    uint32_t radius;                    // R, as bits
+};
+
+// Stages the `count` (even) triangles. The whole block calls it; ends with a
+// block barrier.
+__device__ __forceinline__ void stage_tiny(TinyStage& s, const float* __restrict__ verts,
                                            const uint32_t* __restrict__ perm, uint32_t count) {
+    if (threadIdx.x == 0) s.radius = 0u;
+    __syncthreads();
     for (uint32_t j = threadIdx.x; j < count; j += blockDim.x) {
         const float* q = verts + (size_t)j * 9;
-        s_tri[3 * j] = make_float4(q[0], q[3], q[6], __uint_as_float(perm[j]));
-        s_tri[3 * j + 1] = make_float4(q[1] - q[0], q[4] - q[3], q[7] - q[6], 0.0f);
-        s_tri[3 * j + 2] = make_float4(q[2] - q[0], q[5] - q[3], q[8] - q[6], 0.0f);
+        const f3 v1 = mk3(q[0], q[3], q[6]), v2 = mk3(q[1], q[4], q[7]), v3 = mk3(q[2], q[5], q[8]);
+        const f3 e1 = v2 - v1, e2 = v3 - v1;
+        s.tri[3 * j] = make_float4(v1.x, v1.y, v1.z, __uint_as_float(perm[j]));
+        s.tri[3 * j + 1] = make_float4(e1.x, e1.y, e1.z, 0.0f);
+        s.tri[3 * j + 2] = make_float4(e2.x, e2.y, e2.z, 0.0f);
+        const float r = sqrtf(fmaxf(fmaxf(dot(v1, v1), dot(v2, v2)), dot(v3, v3)));
+        float c[16];
+        const f3 n = cross(e2, e1), c2 = cross(v1, e2), c1 = -cross(v1, e1);
+        c[0] = n.x; c[1] = n.y; c[2] = n.z;
+        c[3] = e2.x; c[4] = e2.y; c[5] = e2.z;
+        c[6] = c2.x; c[7] = c2.y; c[8] = c2.z;
+        c[9] = -e1.x; c[10] = -e1.y; c[11] = -e1.z;
+        c[12] = c1.x; c[13] = c1.y; c[14] = c1.z;
+        c[15] = sqrtf(fmaxf(dot(e1, e1), dot(e2, e2)));
+        const bool usable = r < 1.0e12f;       // far from overflow; otherwise the triangle is always kept
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            reinterpret_cast<float*>(&s.pre[j >> 1][k])[j & 1u] = usable ? c[k] : (k == 15 ? 1.0f : 0.0f);
+        if (usable) atomicMax(&s.radius, __float_as_uint(r));
     }
+    __syncthreads();
 }
 
-__device__ __forceinline__ bool tiny_tri(const float4* __restrict__ tris, uint32_t j, const f3& pos, const f3& dir,
-                                         float& t, uint32_t& id) {
-    const float4 a = tris[3 * j], b = tris[3 * j + 1], c = tris[3 * j + 2];
+#ifdef __CUDACC__
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+#else
+static inline unsigned long long pack2(float a, float b) {
+    return (unsigned long long)float_bits(a) | ((unsigned long long)float_bits(b) << 32);
+}
+static inline float2 unpack2(unsigned long long v) {
+    return make_float2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+}
+static inline unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    const float2 x = unpack2(a), y = unpack2(b), z = unpack2(c);
+    return pack2(__fmaf_rn(x.x, y.x, z.x), __fmaf_rn(x.y, y.y, z.y));
+}
+#endif
+
+// Bit j: triangle j is kept.
+__device__ __forceinline__ uint64_t tiny_filter(const TinyStage& s, uint32_t count, const f3& pos, const f3& dir) {
+    const uint64_t all = count >= 64u ? ~0ull : (1ull << count) - 1ull;
+    const float scale = 4.0e-6f * (sqrtf(dot(pos, pos)) + __uint_as_float(s.radius)) * sqrtf(dot(dir, dir));
+    if (!(scale < 1.0e24f)) return all;
+    const f3 m = cross(pos, dir);
+    const unsigned long long dx = pack2(dir.x, dir.x), dy = pack2(dir.y, dir.y), dz = pack2(dir.z, dir.z);
+    const unsigned long long mx = pack2(m.x, m.x), my = pack2(m.y, m.y), mz = pack2(m.z, m.z);
+    const unsigned long long sc = pack2(scale, scale), one = pack2(-1.0f, -1.0f), zero = pack2(0.0f, 0.0f);
+    uint32_t lo = 0, hi = 0;      // verdicts of the even and the odd triangles, the last pair in bit 0 (0: kept)
+#pragma unroll 1
+    for (uint32_t p = 0; p < count / 2u; ++p) {
+        const ulonglong2* c = reinterpret_cast<const ulonglong2*>(s.pre[p]);
+        const ulonglong2 q0 = c[0], q1 = c[1], q2 = c[2], q3 = c[3], q4 = c[4], q5 = c[5], q6 = c[6], q7 = c[7];
+        const unsigned long long g = fma2(q7.y, sc, zero);
+        const unsigned long long det = fma2(q0.x, dx, fma2(q0.y, dy, fma2(q1.x, dz, fma2(q7.y, sc, g))));
+        const unsigned long long du =
+            fma2(q1.y, mx, fma2(q2.x, my, fma2(q2.y, mz, fma2(q3.x, dx, fma2(q3.y, dy, fma2(q4.x, dz, g))))));
+        const unsigned long long dv =
+            fma2(q4.y, mx, fma2(q5.x, my, fma2(q5.y, mz, fma2(q6.x, dx, fma2(q6.y, dy, fma2(q7.x, dz, g))))));
+        // det - du - dv with a margin of 3 (the terms carry 2, 1 and 1)
+        const unsigned long long w = fma2(dv, one, fma2(du, one, fma2(g, pack2(3.0f, 3.0f), det)));
+        const float2 a = unpack2(det), b = unpack2(du), d = unpack2(dv), e = unpack2(w);
+        lo = __funnelshift_l(__float_as_uint(fminf(min3f(a.x, b.x, d.x), e.x)), lo, 1);
+        hi = __funnelshift_l(__float_as_uint(fminf(min3f(a.y, b.y, d.y), e.y)), hi, 1);
+    }
+    // pair p's verdicts are bit count / 2 - 1 - p: reversed, then interleaved
+    const uint32_t even = __brev(~lo) >> (32u - count / 2u), odd = __brev(~hi) >> (32u - count / 2u);
+    uint64_t mask = 0;
+    auto spread = [](uint32_t x) {
+        uint64_t v = x;
+        v = (v | (v << 16)) & 0x0000FFFF0000FFFFull;
+        v = (v | (v << 8)) & 0x00FF00FF00FF00FFull;
+        v = (v | (v << 4)) & 0x0F0F0F0F0F0F0F0Full;
+        v = (v | (v << 2)) & 0x3333333333333333ull;
+        return (v | (v << 1)) & 0x5555555555555555ull;
+    };
+    mask = spread(even) | (spread(odd) << 1);
+    return mask & all;
+}
+
+__device__ __forceinline__ bool tiny_tri(const TinyStage& s, uint32_t j, const f3& pos, const f3& dir, float& t,
+                                         uint32_t& id) {
+    const float4 a = s.tri[3 * j], b = s.tri[3 * j + 1], c = s.tri[3 * j + 2];
     float u, v;
     id = __float_as_uint(a.w);
     return intersect_tri(pos, dir, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), mk3(c.x, c.y, c.z), u, v, t) && t > kEpsilon;
 }
 
-__device__ __forceinline__ void tiny_closest(const float4* __restrict__ tris, uint32_t count, const f3& pos,
-                                             const f3& dir, float tmax, WideHit& h) {
+__device__ __forceinline__ void tiny_closest(const TinyStage& s, uint32_t count, const f3& pos, const f3& dir,
+                                             float tmax, WideHit& h) {
     h.t = h.t2 = tmax;
     h.best = kNoPrim;
     uint32_t best_id = 0;
-    for (uint32_t j = 0; j < count; ++j) {
+    for (uint64_t kept = tiny_filter(s, count, pos, dir); kept; kept &= kept - 1ull) {
+        const uint32_t j = (uint32_t)__ffsll((long long)kept) - 1u;
         float t;
         uint32_t id;
-        if (!tiny_tri(tris, j, pos, dir, t, id)) continue;
+        if (!tiny_tri(s, j, pos, dir, t, id)) continue;
         if (t < h.t) {
             h.t2 = h.t;
             h.t = t;
@@ -658,17 +767,16 @@ __device__ __forceinline__ void tiny_closest(const float4* __restrict__ tris, ui
     }
 }
 
-__device__ __forceinline__ uint32_t tiny_any(const float4* __restrict__ tris, uint32_t count, const f3& pos,
-                                             const f3& dir, float tmax) {
-    for (uint32_t j = 0; j < count; ++j) {
+__device__ __forceinline__ uint32_t tiny_any(const TinyStage& s, uint32_t count, const f3& pos, const f3& dir,
+                                             float tmax) {
+    for (uint64_t kept = tiny_filter(s, count, pos, dir); kept; kept &= kept - 1ull) {
+        const uint32_t j = (uint32_t)__ffsll((long long)kept) - 1u;
         float t;
         uint32_t id;
-        if (tiny_tri(tris, j, pos, dir, t, id) && t < tmax) return j;
+        if (tiny_tri(s, j, pos, dir, t, id) && t < tmax) return j;
     }
     return kNoPrim;
 }
-#endif  // __CUDACC__
-
 // ------------------------------------------------------------ the checks
 // intersect() visits a triangle's node when the ray's range, clipped by the
 // slab of every node from the root down to it (ray.cuh:225-237), is not empty

@@ -20,16 +20,16 @@ namespace aur {
 namespace {
 
 constexpr int kRenderThreads = 128;
-// Resident blocks per SM that the fused sample kernel is compiled for: its
-// lanes diverge, so what helps is more warps to switch between, even at the
-// price of spills. Measured among 4 to 16: tiny scenes, path mode 1.16-1.30 ms
-// at 4 to 10 and 1.14 at 14 (256x256 box, 16 samples); MIS 1.50-1.59 and 1.44
-// (301x233 emissive box, 9 samples); trees, path mode 1.88 at 8, 1.91 at 6 and
-// 10, 1.94 at 14 (200k-triangle spheres); MIS 2.41 at 6 to 8, 2.35 at 14
-// (4130-triangle box). The per-tile kernel (k_raytrace_mc) runs grids of one
-// 65,536-ray tile, too small for occupancy to matter, and is left
-// unconstrained (a cap made it slower).
-constexpr int render_blocks(bool mis, bool tiny) { return mis || tiny ? 14 : 8; }
+// Resident blocks per SM that the fused sample kernel is compiled for,
+// measured among 4 to 16. Trees: path mode 1.88 ms at 8, 1.91 at 6 and 10, 1.94
+// at 14 (200k-triangle spheres); the MIS estimator 2.41 at 6 to 8, 2.35 at 14
+// (4130-triangle box; its lanes diverge, and more warps to switch between pay
+// for the spills). Tiny scenes: 0.86 ms at 6 and 7, 0.88 at 5 and 8, 0.92 at 14
+// (256x256 box, 16 samples); the MIS estimator 1.14 at 5 and 7, 1.18 at 8 and
+// 14 (301x233 emissive box, 9 samples). The per-tile kernel (k_raytrace_mc)
+// runs grids of one 65,536-ray tile, too small for occupancy to matter, and is
+// left unconstrained (a cap made it slower).
+constexpr int render_blocks(bool mis, bool tiny) { return tiny ? 7 : (mis ? 14 : 8); }
 
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 

@@ -300,10 +300,9 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_tiny(WideView w, uint32
                                                               const float4* __restrict__ rays, uint32_t n,
                                                               float4* __restrict__ hits, uint32_t* __restrict__ occ,
                                                               uint32_t* __restrict__ ctr) {
-    __shared__ float4 s_tri[3 * kTinyTris];
+    __shared__ __align__(16) TinyStage s_stage;
     __shared__ uint8_t s_rank[8][kTinyTris / 2];
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[2] = 0u;  // no chunk is deferred
-    stage_tiny(s_tri, w.verts, w.perm, count);
     if (kAny) {
         for (uint32_t j = threadIdx.x; j < 8u * w.nodes; j += blockDim.x) {
             const uint32_t oct = j & 7u, node = j >> 3, lvl = 31u - (uint32_t)__clz(node + 1u);
@@ -320,7 +319,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_tiny(WideView w, uint32
             s_rank[oct][node] = (uint8_t)rank;
         }
     }
-    __syncthreads();
+    stage_tiny(s_stage, w.verts, w.perm, count);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 r0 = rays[2 * (size_t)i];
@@ -334,15 +333,16 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_tiny(WideView w, uint32
     if (kAny) {
         const uint32_t oct = dir_octant(r.dir);
         uint32_t first = ~0u;
-        for (uint32_t j = 0; j < count; ++j) {
+        for (uint64_t kept = tiny_filter(s_stage, count, r.pos, r.dir); kept; kept &= kept - 1ull) {
+            const uint32_t j = (uint32_t)__ffsll((long long)kept) - 1u;
             float t;
             uint32_t id;
-            if (tiny_tri(s_tri, j, r.pos, r.dir, t, id) && t < r0.w)
+            if (tiny_tri(s_stage, j, r.pos, r.dir, t, id) && t < r0.w)
                 first = min(first, ((uint32_t)s_rank[oct][j >> 1] << 8) | j);
         }
         if (first != ~0u) h.best = first & 255u;
     } else {
-        tiny_closest(s_tri, count, r.pos, r.dir, r0.w, h);
+        tiny_closest(s_stage, count, r.pos, r.dir, r0.w, h);
     }
     float u = 0.0f, v = 0.0f;
     if (kAny) h.best = finish_any(w, r, h.best, r0.w);

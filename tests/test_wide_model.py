@@ -61,15 +61,15 @@ def _check(lib, V, rays):
     tuv, prim, steps = np.zeros((n, 3), np.float32), np.zeros(n, np.uint32), np.zeros(n, np.uint32)
     changed = []
     try:
-        for mode in range(3):
+        for mode in range(5 if len(perm) <= 64 else 3):
             changed.append(lib.wide_model_trace(m, rays.ctypes.data, n, mode, tuv.ctypes.data, prim.ctypes.data,
                                                 steps.ctypes.data))
             assert changed[-1] >= 0, "the traversal does not end"
-            if mode == 0:
+            if mode in (0, 3):
                 assert np.array_equal(prim, ohits["prim"])
                 for q, f in enumerate("tuv"):
                     assert np.array_equal(tuv[:, q].view(np.uint32), ohits[f].view(np.uint32)), f
-            elif mode == 1:
+            elif mode in (1, 4):
                 assert np.array_equal(prim, (oocc != T.NO_HIT).astype(np.uint32))
             else:
                 assert np.array_equal(prim, oocc)
@@ -146,6 +146,26 @@ def test_lattice_planes(model):
     d[np.all(d == 0, axis=1)] = (1.0, 0.0, 0.0)
     _check(model, V.reshape(-1, 9), _rays(o, d))
     _check(model, V.reshape(-1, 9), _rays(o, d / np.linalg.norm(d, axis=1, keepdims=True)))
+
+
+@pytest.mark.parametrize("n_tris", [2, 33, 64])
+@pytest.mark.parametrize("scale,shift", [(1.0, 0.0), (1.0, 1000.0), (1e-4, 0.0), (1e4, -3e5), (1e13, 0.0), (1e18, 1e19)])
+def test_few_triangles_over_coordinate_ranges(model, n_tris, scale, shift):
+    """Edges, vertices and grazing rays of a few triangles: the filter in front
+    of the exact tests keeps every triangle they accept."""
+    rng = np.random.default_rng(n_tris)
+    V = (rng.random((n_tris, 3, 1)) + rng.normal(size=(n_tris, 3, 3)) * 0.3) * scale + shift
+    V = V.astype(np.float32)
+    P = V[rng.integers(0, n_tris, 3000)].astype(np.float64)      # triangle, axis, corner
+    a, b = rng.random((2, 3000))
+    a[:1000] = np.round(a[:1000])                                  # on edges and vertices
+    b = b * (1 - a)
+    target = P[:, :, 0] + a[:, None] * (P[:, :, 1] - P[:, :, 0]) + b[:, None] * (P[:, :, 2] - P[:, :, 0])
+    o = target + rng.normal(size=(3000, 3)) * scale * rng.choice([1e-3, 1.0, 100.0], (3000, 1))
+    e = P[:, :, 1] - P[:, :, 0]
+    o[2000:] = target[2000:] - e[2000:] + 1e-4 * (o[2000:] - target[2000:])
+    d = target - o
+    _check(model, V.reshape(-1, 9), _rays(o, d / np.linalg.norm(d, axis=1, keepdims=True), 1.0e30))
 
 
 @pytest.mark.parametrize("scale,shift", [(1.0, 1000.0), (1e-3, 0.0), (1e4, -3e4), (1e-6, 1.0), (1e18, 0.0)])

@@ -33,6 +33,11 @@ static inline uint32_t __byte_perm(uint32_t x, uint32_t y, uint32_t s) {
     return r;
 }
 static inline uint32_t __funnelshift_l(uint32_t lo, uint32_t hi, uint32_t s) { return s ? (hi << s) | (lo >> (32 - s)) : hi; }
+static inline uint32_t __brev(uint32_t x) { uint32_t r = 0; for (int i = 0; i < 32; ++i) r |= ((x >> i) & 1u) << (31 - i); return r; }
+/* one thread that plays a whole block */
+static const struct { uint32_t x; } threadIdx = {0}, blockDim = {1};
+#define __syncthreads()
+static inline void atomicMax(uint32_t* p, uint32_t v) { if (v > *p) *p = v; }
 #define __shfl_xor_sync(m, v, o) (v)
 #define __any_sync(m, p) (p)
 #define __reduce_or_sync(m, v) (v)
@@ -102,7 +107,8 @@ void* wide_model_create(const float* verts, const uint32_t* perm, uint32_t count
 void wide_model_destroy(void* p) { delete (Model*)p; }
 
 /* mode 0: closest hit (t, u, v, prim id) per ray; 1: any hit, 1 or 0 in
- * prim; 2: the occluder intersectAny() reports. Rays are 8 floats (origin,
+ * prim; 2: the occluder intersectAny() reports; 3, 4: modes 0 and 1 without
+ * the tree (at most kTinyTris triangles). Rays are 8 floats (origin,
  * tmax, direction, pad). steps[i] (optional): treelet steps of ray i.
  * Returns the number of rays that left the treelets for the exact walk's
  * checks to reject, or -1 when a ray took more steps than there are items. */
@@ -110,18 +116,28 @@ long wide_model_trace(void* p, const float* rays, uint32_t n, int mode, float* t
     Model* m = (Model*)p;
     const WideView w{m->recs.data(), m->wide.data(), m->perm.data(), m->verts.data(), m->n, m->levels};
     long changed = 0;
+    TinyStage* tiny = nullptr;
+    if (mode >= 3) {
+        if (2 * m->n > kTinyTris) return -1;
+        tiny = new TinyStage;
+        stage_tiny(*tiny, m->verts.data(), m->perm.data(), 2 * m->n);
+    }
     for (uint32_t i = 0; i < n; ++i) {
         const float* q = rays + 8 * (size_t)i;
         WideRay r;
         WideState s;
         WideHit h;
         uint64_t c = 1;
-        if (wide_begin(r, s, h, w, mk3(q[0], q[1], q[2]), mk3(q[4], q[5], q[6]), q[3])) while (mode == 0 ? wide_step<kWideClosest>(w, r, s, h) : mode == 1 ? wide_step<kWideAny>(w, r, s, h) : wide_step<kWideFirst>(w, r, s, h))
+        const f3 pos = mk3(q[0], q[1], q[2]), dir = mk3(q[4], q[5], q[6]);
+        const bool begun = wide_begin(r, s, h, w, pos, dir, q[3]);
+        if (mode == 3) tiny_closest(*tiny, 2 * m->n, pos, dir, q[3], h);
+        else if (mode == 4) h.best = tiny_any(*tiny, 2 * m->n, pos, dir, q[3]);
+        else if (begun) while (mode == 0 ? wide_step<kWideClosest>(w, r, s, h) : mode == 1 ? wide_step<kWideAny>(w, r, s, h) : wide_step<kWideFirst>(w, r, s, h))
             if (++c > 3ull * m->n + 8) return -1;
         if (steps) steps[i] = (uint32_t)c;
         const uint32_t found = h.best;
         float u = 0, v = 0;
-        if (mode == 0) {
+        if (mode == 0 || mode == 3) {
             finish_closest(w, r, h, q[3], u, v);
             tuv[3 * (size_t)i] = h.best == kNoPrim ? q[3] : h.t;
             tuv[3 * (size_t)i + 1] = h.best == kNoPrim ? 0.0f : u;
@@ -130,8 +146,9 @@ long wide_model_trace(void* p, const float* rays, uint32_t n, int mode, float* t
             h.best = finish_any(w, r, h.best, q[3]);
         }
         changed += found != h.best;
-        prim[i] = mode == 1 ? (h.best != kNoPrim) : h.best == kNoPrim ? 0xFFFFFFFFu : m->perm[h.best];
+        prim[i] = mode == 1 || mode == 4 ? (h.best != kNoPrim) : h.best == kNoPrim ? 0xFFFFFFFFu : m->perm[h.best];
     }
+    delete tiny;
     return changed;
 }
 
