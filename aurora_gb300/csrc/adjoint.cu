@@ -35,9 +35,6 @@
 #include <type_traits>
 #include <vector>
 
-#include <cooperative_groups.h>
-#include <cooperative_groups/reduce.h>
-
 #include "aur_integrate.cuh"
 #include "aur_internal.h"
 
@@ -45,11 +42,14 @@ namespace aur {
 namespace {
 
 constexpr int kAdjThreads = 128;
-// The replay kernel is compiled for 14 resident blocks per SM (at most 36
-// registers, spills served by L1): its lanes diverge and it waits on latency,
-// so more warps pay for the spills. 256x256, 16 samples of the 4130-triangle
-// box: 6.1 ms at 8 blocks, 5.9 at 10, 5.8 at 12, 5.3 at 14 and 16.
-constexpr int kAdjBlocksPerSm = 14;
+// Resident blocks per SM that the replay kernel is compiled for: its lanes
+// diverge and it waits on latency and instruction fetch, so more warps pay for
+// the spills. With per-warp sums (256x256, 16 samples of a 4130-triangle box
+// with a shader each): 4.75 ms at 6 blocks, 4.49 at 8, 4.33 at 10, 4.35 at 12,
+// 4.42 at 14, in the MIS mode 3.49, 3.41, 3.11, 2.99 and 2.88 (8 samples). With
+// a thread's own sums (100k-triangle spheres, 8 samples): 2.13 ms at 8, 2.14 at
+// 10, 2.25 at 12, 2.53 at 14.
+constexpr int adj_blocks(bool few) { return few ? 10 : 12; }
 constexpr uint32_t kSharedLights = 64;
 
 // Per-unit-colour radiance of a light sample (Lr = color * s), light.cuh:228-259.
@@ -60,58 +60,82 @@ __device__ __forceinline__ float light_scale(const aur_light& L, const f3& dir, 
     return L.intensity * fmaxf(0.0f, dot(from(L.direction), -dir));
 }
 
-// Adds g_c1 * d(colour1)/d(diffuse_color) = g_c1 * diffuse to shader si's
-// gradient (colour1 = diffuse_color * diffuse; a textured shader's colour is
-// not its diffuse_color, so it gets none). Lanes that hit the same shader
-// (large triangles are hit by most of a warp) are summed first, so a warp
-// issues one atomic per shader instead of one per lane.
-__device__ __forceinline__ void add_diffuse_grad(float* __restrict__ d_diffuse, uint32_t si, const aur_shader* sh,
-                                                 const f3& g_c1) {
-    const f3 gd = sh->texture > 0 ? mk3(0.0f) : g_c1 * sh->diffuse;
-    namespace cg = cooperative_groups;
-    const cg::coalesced_group active = cg::coalesced_threads();
-    const cg::coalesced_group same = cg::labeled_partition(active, si);
-    const float sx = cg::reduce(same, gd.x, cg::plus<float>());
-    const float sy = cg::reduce(same, gd.y, cg::plus<float>());
-    const float sz = cg::reduce(same, gd.z, cg::plus<float>());
-    if (same.thread_rank() == 0 && (sx != 0.0f || sy != 0.0f || sz != 0.0f)) {
-        atomicAdd(d_diffuse + 3 * si + 0, sx);
-        atomicAdd(d_diffuse + 3 * si + 1, sy);
-        atomicAdd(d_diffuse + 3 * si + 2, sz);
-    }
-}
+// Where a thread's shader gradients go. kFew (at most kFewShaders shaders):
+// into the thread's own sums, which the block adds up once its samples are
+// done (100k-triangle spheres, eight shaders: 2.65 -> 2.14 ms); else to the
+// result, summed first over the lanes of the warp that hit the same shader
+// (large triangles are hit by most of a warp), one atomic per shader and
+// component. A library reduction per shader group ran the groups one after
+// the other: 5.2 ms on a 4130-triangle box with a shader each, 4.3 ms in
+// rounds over all groups at once.
+constexpr uint32_t kFewShaders = 8;
 
-// Adds g to shader si's entry of a per-shader gradient (emission), summed per
-// warp over the lanes that hit the same shader first.
-__device__ __forceinline__ void add_shader_grad(float* __restrict__ d, uint32_t si, const f3& gs) {
-    namespace cg = cooperative_groups;
-    const cg::coalesced_group active = cg::coalesced_threads();
-    const cg::coalesced_group same = cg::labeled_partition(active, si);
-    const float sx = cg::reduce(same, gs.x, cg::plus<float>());
-    const float sy = cg::reduce(same, gs.y, cg::plus<float>());
-    const float sz = cg::reduce(same, gs.z, cg::plus<float>());
-    if (same.thread_rank() == 0 && (sx != 0.0f || sy != 0.0f || sz != 0.0f)) {
-        atomicAdd(d + 3 * si + 0, sx);
-        atomicAdd(d + 3 * si + 1, sy);
-        atomicAdd(d + 3 * si + 2, sz);
+template <bool kFew>
+struct ShaderGrads {
+    float* diffuse;      // 3 per shader
+    float* emission;     // 3 per shader, or null
+    float sum[kFew ? 6 * kFewShaders : 1];
+
+    __device__ __forceinline__ void clear() {
+        if (kFew)
+            for (uint32_t k = 0; k < 6 * kFewShaders; ++k) sum[k] = 0.0f;
     }
-}
+    // Adds g to shader si's entry.
+    __device__ __forceinline__ void add(bool to_emission, uint32_t si, const f3& g) {
+        if constexpr (kFew) {
+            float* s = sum + (to_emission ? 3 * kFewShaders : 0u) + 3 * si;
+            s[0] += g.x;
+            s[1] += g.y;
+            s[2] += g.z;
+        } else {
+            // lanes of one shader in pairs, neighbours in rank first, all
+            // shaders at once: at most five rounds
+            const uint32_t here = __activemask(), lane = threadIdx.x & 31;
+            const uint32_t peers = __match_any_sync(here, si);
+            uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+            uint32_t above = peers & (0xFFFFFFFEu << lane);
+            const bool first = rank == 0;
+            f3 x = g;
+            while (__any_sync(here, above != 0u)) {
+                const int next = __ffs(above);
+                const int src = next ? next - 1 : (int)lane;
+                const float ax = __shfl_sync(here, x.x, src), ay = __shfl_sync(here, x.y, src),
+                            az = __shfl_sync(here, x.z, src);
+                if (next) x = x + mk3(ax, ay, az);
+                above &= __ballot_sync(here, !(rank & 1u));
+                rank >>= 1;
+            }
+            if (first && (x.x != 0.0f || x.y != 0.0f || x.z != 0.0f)) {
+                float* d = (to_emission ? emission : diffuse) + 3 * (size_t)si;
+                atomicAdd(d + 0, x.x);
+                atomicAdd(d + 1, x.y);
+                atomicAdd(d + 2, x.z);
+            }
+        }
+    }
+    // Adds g_c1 * d(colour1)/d(diffuse_color) = g_c1 * diffuse to shader si's
+    // gradient (colour1 = diffuse_color * diffuse; a textured shader's colour
+    // is not its diffuse_color, so it gets none).
+    __device__ __forceinline__ void add_diffuse(uint32_t si, const aur_shader* sh, const f3& g_c1) {
+        add(false, si, sh->texture > 0 ? mk3(0.0f) : g_c1 * sh->diffuse);
+    }
+};
 
 // Direct light at a hit as the primal computes it (direct_light), with its
 // derivatives: Dp receives the direct light per unit Lambert colour, and the
 // light-colour gradients g * thr * d(direct)/d(colour_l) are added (light 0
 // into gl0, the others to d_light). ew: the emission's MIS weight; bounce:
 // whether a diffuse bounce follows the hit (both for AUR_MODE_PATH_MIS).
-// With d_emission, the emission gradients of the hit's own shader si and of
+// With an emission result, the emission gradients of the hit's own shader si and of
 // the emitter sample's shader are added too.
-template <bool kMis, typename Trav>
+template <bool kMis, typename Trav, typename Grads>
 __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader* sh, const Bsdf& b, const f3& f,
                                           const f3& position, const f3& wo, float ew, bool bounce, uint32_t seed,
                                           uint32_t scene, uint32_t pixel, uint32_t sample, uint32_t rix, const f3& thr,
                                           const f3& g, float* __restrict__ d_light, f3& gl0, f3& Dp,
-                                          float* __restrict__ d_emission, uint32_t si, const Trav& trav, uint32_t* err) {
+                                          Grads& grads, uint32_t si, const Trav& trav, uint32_t* err) {
     f3 Li = kMis ? from(sh->emission_color) * ew : from(sh->emission_color);
-    if (d_emission) add_shader_grad(d_emission, si, kMis ? (g * thr) * ew : g * thr);
+    if (grads.emission) grads.add(true, si, kMis ? (g * thr) * ew : g * thr);
     Dp = mk3(0.0f);   // direct light per unit Lambert colour
     for (uint32_t i = 0; i < sc.num_lights; ++i) {
         const aur_light& L = sc.lights[i];
@@ -203,7 +227,7 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
         const bool vis = ss.cand && !occluded(sc, trav, ss.o, ss.d, tt);
         Li = Li + (vis ? ss.c : mk3(0.0f));
         if (vis) Dp = Dp + ss.e * (ss.geo * kInvPi);
-        if (d_emission && vis) add_shader_grad(d_emission, ss.esi, (g * thr) * (f * ss.geo));
+        if (grads.emission && vis) grads.add(true, ss.esi, (g * thr) * (f * ss.geo));
     }
     return Li;
 }
@@ -224,11 +248,10 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
 // colour and in the light colour. One pass replaces a primal pass (each
 // sample's radiance) plus a replay: 29.3 -> 21.1 ms on the differentiable
 // workload (256x256, 64 spp, path mode).
-template <bool kMis, typename Trav>
+template <bool kMis, typename Trav, typename Grads>
 __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t mode, uint32_t seed, uint32_t scene,
                              uint32_t pixel, uint32_t sample, const PathRay& primary, const Trav& trav,
-                             const f3& g, float* __restrict__ d_diffuse, float* __restrict__ d_light,
-                             float* __restrict__ d_emission, f3& gl0, uint32_t* err) {
+                             const f3& g, Grads& grads, float* __restrict__ d_light, f3& gl0, uint32_t* err) {
     struct Marker {
         f3 col0, c1;          // colour before the subtree, the bouncing vertex's Lambert colour
         const aur_shader* sh;
@@ -250,7 +273,7 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
         dc.x = m.c1.x != 0.0f ? sub.x / m.c1.x : 0.0f;
         dc.y = m.c1.y != 0.0f ? sub.y / m.c1.y : 0.0f;
         dc.z = m.c1.z != 0.0f ? sub.z / m.c1.z : 0.0f;
-        add_diffuse_grad(d_diffuse, m.si, m.sh, g * dc);
+        grads.add_diffuse(m.si, m.sh, g * dc);
     };
     for (;;) {
         while (nm > 0 && sp <= mk[nm - 1].base) close(mk[--nm]);
@@ -278,8 +301,8 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
             continue_ray<kMis>(sh, b, cur, position, wo, path, depth, maxd, seed, scene, pixel, sample, rix);
         f3 Dp;
         const f3 Li = direct_grad<kMis>(sc, sh, b, f, position, wo, ew, bounce_follows, seed, scene, pixel, sample, rix,
-                                        cur.thr, g, d_light, gl0, Dp, d_emission, si, trav, err);
-        add_diffuse_grad(d_diffuse, si, sh, g * (cur.thr * Dp));
+                                        cur.thr, g, d_light, gl0, Dp, grads, si, trav, err);
+        grads.add_diffuse(si, sh, g * (cur.thr * Dp));
         col = col + Li * cur.thr;
         for (int q = 0; q < kc.n; ++q) {
             if (kc.bounced && q == kc.n - 1) {   // the diffuse bounce: its subtree scales with this vertex's colour
@@ -297,15 +320,16 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
     while (nm > 0) close(mk[--nm]);
 }
 
-// Replay kernel: one thread per camera sample of samples [s0, s0 + nb).
-template <bool kMis, bool kTiny>
-__global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) k_adj_replay(SceneView sc, aur_camera cam,
+// Replay kernel: one thread per camera sample of samples [s0, s0 + nb). kFew: at most kFewShaders shaders.
+template <bool kMis, bool kTiny, bool kFew>
+__global__ void __launch_bounds__(kAdjThreads, adj_blocks(kFew)) k_adj_replay(SceneView sc, aur_camera cam,
                                                                             aur_render_params p, uint32_t s0,
                                                                             uint32_t nb,
                                                                             const float4* __restrict__ d_image,
                                                                             float* __restrict__ d_diffuse,
                                                                             float* __restrict__ d_light,
                                                                             float* __restrict__ d_emission,
+                                                                            uint32_t shaders,
                                                                             uint32_t* __restrict__ err) {
     const auto trav = make_trav<kTiny>(sc);
     __shared__ float s_light[3 * kSharedLights];
@@ -315,8 +339,12 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) k_adj_replay(Sce
         for (uint32_t i = threadIdx.x; i < 3 * sc.num_lights; i += kAdjThreads) s_light[i] = 0.0f;
     __syncthreads();
     const uint64_t P = (uint64_t)p.width * p.height;
-    const uint64_t t = (uint64_t)blockIdx.x * kAdjThreads + threadIdx.x;
     f3 gl0 = mk3(0.0f);
+    ShaderGrads<kFew> grads;
+    grads.diffuse = d_diffuse;
+    grads.emission = d_emission;
+    grads.clear();
+    const uint64_t t = (uint64_t)blockIdx.x * kAdjThreads + threadIdx.x;
     if (t < P * nb) {
         const uint32_t pix = (uint32_t)(t % P);
         const uint32_t s = s0 + (uint32_t)(t / P);
@@ -324,8 +352,26 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) k_adj_replay(Sce
         const float4 di = d_image[pix];
         const float w = 1.0f / (float)p.spp;
         const f3 g = mk3(di.x * w, di.y * w, di.z * w);
-        replay_stack<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, d_diffuse,
-                           shared_lights ? s_light : d_light, d_emission, gl0, err);
+        replay_stack<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, grads,
+                           shared_lights ? s_light : d_light, gl0, err);
+    }
+    if constexpr (kFew) {      // the block's sums, one atomic per entry
+        __shared__ float s_sum[kAdjThreads / 32][6 * kFewShaders];
+        const uint32_t lane = threadIdx.x & 31;
+        for (uint32_t k = 0; k < 6 * kFewShaders; ++k) {
+            float x = grads.sum[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (lane == 0) s_sum[threadIdx.x >> 5][k] = x;
+        }
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < 6 * kFewShaders; k += kAdjThreads) {
+            const bool em = k >= 3 * kFewShaders;
+            const uint32_t e = em ? k - 3 * kFewShaders : k;
+            float x = 0.0f;
+            for (int q = 0; q < kAdjThreads / 32; ++q) x += s_sum[q][k];
+            if (e < 3 * shaders && x != 0.0f && (!em || d_emission)) atomicAdd((em ? d_emission : d_diffuse) + e, x);
+        }
     }
     // light 0: warp sum, then one shared atomic per warp
 #pragma unroll
@@ -385,13 +431,17 @@ aur_status aur_render_adjoint(aur_ctx* ctx, const aur_scene* scene, const aur_ca
     for (uint32_t s = s0; s < s1; s += batch) {
         const uint32_t nb = std::min(batch, s1 - s);
         const uint32_t grid = cdiv(P * nb, kAdjThreads);
-        auto go = [&](auto m, auto tiny) {
-            k_adj_replay<m.value, tiny.value><<<grid, kAdjThreads, 0, ctx->stream>>>(
-                sv, *camera, p, s, nb, di, d_diffuse, d_light_color, d_emission, ctx->d_flags);
+        auto go = [&](auto m, auto tiny, auto few) {
+            k_adj_replay<m.value, tiny.value, few.value><<<grid, kAdjThreads, 0, ctx->stream>>>(
+                sv, *camera, p, s, nb, di, d_diffuse, d_light_color, d_emission, scene->num_shaders, ctx->d_flags);
+        };
+        auto pick = [&](auto m, auto tiny) {
+            if (scene->num_shaders <= kFewShaders) go(m, tiny, std::true_type{});
+            else go(m, tiny, std::false_type{});
         };
         const bool tiny = scene->nmh->count <= kTinyTris;
-        if (mis) tiny ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
-        else tiny ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
+        if (mis) tiny ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
+        else tiny ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{});
     }
     AUR_CUDA(cudaGetLastError());
     return AUR_OK;
