@@ -40,7 +40,11 @@ constexpr uint32_t kDone = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
 constexpr int kTileItems = 16;                       // per thread, scan tiles
 constexpr uint32_t kTile = kThreads * kTileItems;     // 4096
-constexpr int kSelectItems = 16;                     // per thread, k_select (a multiple of 4)
+// k_select's list entries per thread (multiples of 4): few where the list is
+// too short to fill the GPU with many. 100k triangles 375 us (4) against 421
+// (16), 250k 446 against 482, 1M 1016 against 1005.
+constexpr int kSelectItems = 16, kSelectFew = 4;
+constexpr uint32_t kSelectShort = 1u << 19;
 constexpr int kSortItems = 8;
 constexpr uint32_t kSortTile = kThreads * kSortItems; // 2048
 
@@ -306,7 +310,8 @@ __device__ __forceinline__ bool build_aborted(const uint32_t* err) {
 // Segmented arg-max of (max-key, lowest prim id) over each node's segment,
 // excluding the segment's first element, which is recorded as pair[0]
 // (swapMaxTriangleTPS/TPT, rebuilder.cu:93-151). Each thread owns
-// kSelectItems consecutive list positions.
+// kItems consecutive list positions.
+template <int kItems>
 __global__ void __launch_bounds__(kThreads) k_select(const uint32_t* __restrict__ list, uint32_t M,
                                                      const float* __restrict__ mxa,
                                                      const uint32_t* __restrict__ node_of,
@@ -315,30 +320,30 @@ __global__ void __launch_bounds__(kThreads) k_select(const uint32_t* __restrict_
                                                      uint32_t* __restrict__ heap, uint32_t* node_of_out,
                                                      uint32_t* __restrict__ done, const uint32_t* err) {
     if (build_aborted(err)) return;       // whole blocks: the word does not change during this launch
-    const uint32_t base = (blockIdx.x * kThreads + threadIdx.x) * kSelectItems;
+    const uint32_t base = (blockIdx.x * kThreads + threadIdx.x) * kItems;
     const int lane = threadIdx.x & 31;
     uint32_t cur = kDone;
     unsigned long long cur_key = 0;
     bool first_run = true;
     if (base < M) {
-        const int cnt = (M - base) < (uint32_t)kSelectItems ? (int)(M - base) : kSelectItems;
-        uint32_t pid[kSelectItems];
-        if (cnt == kSelectItems) {
+        const int cnt = (M - base) < (uint32_t)kItems ? (int)(M - base) : kItems;
+        uint32_t pid[kItems];
+        if (cnt == kItems) {
             const uint4* p = reinterpret_cast<const uint4*>(list + base);
 #pragma unroll
-            for (int q = 0; q < kSelectItems / 4; ++q) {
+            for (int q = 0; q < kItems / 4; ++q) {
                 const uint4 v = p[q];
                 pid[4 * q] = v.x; pid[4 * q + 1] = v.y; pid[4 * q + 2] = v.z; pid[4 * q + 3] = v.w;
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < kSelectItems; ++i) pid[i] = i < cnt ? list[base + i] : 0u;
+            for (int i = 0; i < kItems; ++i) pid[i] = i < cnt ? list[base + i] : 0u;
         }
-        uint32_t nd[kSelectItems];
+        uint32_t nd[kItems];
 #pragma unroll
-        for (int i = 0; i < kSelectItems; ++i) nd[i] = i < cnt ? node_of[pid[i]] : kDone;
+        for (int i = 0; i < kItems; ++i) nd[i] = i < cnt ? node_of[pid[i]] : kDone;
 #pragma unroll
-        for (int i = 0; i < kSelectItems; ++i) {
+        for (int i = 0; i < kItems; ++i) {
             if (i >= cnt) break;
             const uint32_t k = nd[i];
             unsigned long long key;
@@ -1357,9 +1362,13 @@ void enqueue_build(Seq& q, const BuildArgs& b) {
         const uint32_t mt = cdiv(M, kTile);
         // each node's pair: its segment's first entry and the entry of largest max-key
         unsigned long long* lb = tiles + lv * (lookback_bytes(ntiles) / sizeof(unsigned long long));
-        q.launch(k_select, dim3(cdiv(M, (uint32_t)kThreads * kSelectItems)), dim3(kThreads), 0, listA + a * S, M,
-                 mx + a * S, node_of, ns, L0, L1, best, pair0, heap, node_of,
-                 reinterpret_cast<uint32_t*>(lb + 3 * ntiles) + 3, b.flags);
+        auto select = [&](auto kernel, uint32_t items) {
+            q.launch(kernel, dim3(cdiv(M, (uint32_t)kThreads * items)), dim3(kThreads), 0, listA + a * S, M, mx + a * S,
+                     node_of, ns, L0, L1, best, pair0, heap, node_of, reinterpret_cast<uint32_t*>(lb + 3 * ntiles) + 3,
+                     b.flags);
+        };
+        if (M <= kSelectShort) select(k_select<kSelectFew>, kSelectFew);
+        else select(k_select<kSelectItems>, kSelectItems);
         if (lv + 1 == levels) break;
         ListSet sb;
         sb.in[0] = listA + bx * S; sb.out[0] = listB + bx * S;
