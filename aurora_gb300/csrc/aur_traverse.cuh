@@ -118,9 +118,8 @@ __device__ __forceinline__ Sector ld_sector(const float4* __restrict__ p) {
 }
 
 // The same sector with two 16-byte loads, for the walks of this file: they run
-// where time does not count (the counting kernels, and the treelets' rare
-// fallback, a function that is not inlined: ptxas 13.0 fails on a 256-bit load
-// in one).
+// where time does not count: the counting kernels, and the rare fallback of
+// the treelets' walk.
 __device__ __forceinline__ Sector ld_halves(const float4* __restrict__ p) {
     Sector s;
 #ifdef __CUDACC__

@@ -201,8 +201,8 @@ __global__ void k_radix_scan_rows(uint32_t* __restrict__ hist, uint32_t nb, uint
 // Stable scatter of one radix pass. A warp ranks its 256 consecutive keys
 // against its own digit counts, without a block barrier; the tile is then
 // sorted in shared memory and written out in digit runs, so that neighbouring
-// threads store neighbouring words. (3 x 1M keys: 18 us a pass; a barrier-
-// separated round per 256 keys with scattered stores took 41 us.)
+// threads store neighbouring words. (3 x 1M keys with a cold L2: 28 us a
+// pass; a barrier-separated round per 256 keys with scattered stores took 41.)
 __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* __restrict__ kin,
                                                             const uint32_t* __restrict__ vin,
                                                             uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
@@ -972,7 +972,7 @@ __device__ __forceinline__ void st_sector(float4* p, const float4& a, const floa
 // triangles as (v1, e1, e2), and the padded subtree boxes of the children (an
 // empty box where a child does not exist). The vertices go through shared
 // memory, so that the gather and the copy out walk consecutive words; a record
-// is written as four whole 32-byte sectors. (1M triangles: 45 us; pair order,
+// is written as four whole 32-byte sectors. (1M triangles: 48 us; pair order,
 // vertices with half-written records, and the boxes in ten further launches
 // took 138 us.)
 constexpr uint32_t kEmitNodes = 128;
@@ -1047,7 +1047,7 @@ __global__ void __launch_bounds__(kEmitNodes) k_emit_nodes(const float* __restri
 }
 
 // One thread per treelet writes its record (wide_record) from the NMH-ordered
-// vertices and the subtree boxes of k_local_finish and k_node_boxes.
+// vertices and the subtree boxes of k_local_finish and k_upper_boxes.
 __global__ void __launch_bounds__(128) k_wide_nodes(const float* __restrict__ verts, const float* __restrict__ box,
                                                     uint32_t n, uint32_t levels, uint32_t treelets,
                                                     uint4* __restrict__ wide, const uint32_t* err) {

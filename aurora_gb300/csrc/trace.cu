@@ -187,11 +187,13 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace(const float4* __rest
 // kRefill of them wait. Compiled for 8 blocks per SM (64 registers, none
 // spilled): what bounds it is latency and the issue slots (the box tests'
 // integer pipe), not memory. Per 8M random rays over 1M triangles, closest
-// hit: 4, 6, 7, 8, 9 and 10 blocks per SM 11.3, 10.5, 10.0, 9.5, 9.7 and 10.0
-// ms; refilled at 1, 2, 4, 6 and 8 waiting lanes 10.1, 9.6, 9.3, 9.4 and 9.5
-// ms; triangles tested by the lane that met them instead of the queue 12.2
-// ms; the node-by-node kernel it replaces 18.3 ms. Any hit, 4M rays toward a
-// light: 7.2 ms before, 3.8 ms now.
+// hit, before the packed box tests (wide_step) took 0.5 ms off: 8, 9 and 10
+// blocks per SM 9.3, 9.7 and 10.0 ms (refilled at 8 lanes, 5, 6, 7 and 8
+// blocks: 10.3, 10.5, 10.0 and 9.5); refilled at 1, 2, 4, 6 and 8 waiting
+// lanes 10.1, 9.6, 9.3, 9.4 and 9.5 ms; triangles tested by the lane that met
+// them instead of the queue 12.2 ms. Now 8.8 ms; the node-by-node kernel it
+// replaces took 18.3 ms. Any hit, 4M rays toward a light: 7.2 ms before, 3.7
+// ms now.
 constexpr int kRefill = 4;
 
 template <bool kAny>

@@ -969,7 +969,7 @@ aur_status make_graph(aur_batch* bt) {
         // the previous iteration's shadow rays beside this one's paths: each
         // stage ends with a few long rays, under which the other's run (a
         // 2M-triangle terrain, nine iterations: 22.6 ms one after the other,
-        // 18.9 ms so)
+        // 19.8 ms so)
         AUR_CUDA(cudaEventRecord(bt->fork, s));
         AUR_CUDA(cudaStreamWaitEvent(bt->side_stream, bt->fork, 0));
         launch_shadow(bt, a, bt->side_stream);

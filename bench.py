@@ -48,13 +48,9 @@ sys.path.insert(0, ROOT)
 
 N_TRIS = 1_000_000
 N_RAYS = 1 << 24
-RAY_IN_BYTES = 28      # origin, direction, tmax (this traversal's own reads)
 REF_RAY_IN_BYTES = 24  # origin, direction: the reference algorithm's ray
 HIT_OUT_BYTES = 16     # t, u, v, prim
 NODE_BYTES = 72        # two triangles, as the reference fetches per visited node
-SLAB_BYTES = 16        # first word of a node record: slab lo/hi (+ 8 B of triangle)
-TRI_BYTES = 64         # rest of the two triangles, read when the slab is crossed
-BOX_BYTES = 48         # children's subtree boxes, read before descending
 NMH_LEVEL_BYTES = 32   # NMH build, per triangle per level: 16 B read + 16 B written
 METRIC = "Mrays/s closest-hit"
 WORKLOAD = ("traversal microbench: 1M triangles (centroid U[0,1]^3, edges LogNormal(-4,0.5)), 2^24 rays "
@@ -265,7 +261,7 @@ def load_peaks():
     return 6800.0, "fallback"
 
 
-TRAVERSAL_SOURCES = ("aurora_gb300/csrc/trace.cu", "aurora_gb300/csrc/aur_traverse.cuh",
+TRAVERSAL_SOURCES = ("aurora_gb300/csrc/trace.cu", "aurora_gb300/csrc/aur_wide.cuh", "aurora_gb300/csrc/aur_traverse.cuh",
                      "aurora_gb300/csrc/aur_math.cuh")
 TRAFFIC_PROFILE = "profiles/k_trace_microbench_full.md"
 
@@ -280,7 +276,7 @@ def traversal_source_sha():
 
 
 def load_traffic():
-    """(DRAM bytes of one closest-hit trace, both launches; where they come from).
+    """(DRAM bytes of one closest-hit trace, its launches together; where they come from).
 
     The committed ncu summary holds 'traffic_bytes_per_trace: N' and
     'source_sha256_16: H', H being traversal_source_sha() of the sources it
@@ -996,8 +992,6 @@ def main():
 
     peak, peak_kind = load_peaks()
     wc = work["closest"]
-    own_bytes = (N_RAYS * (RAY_IN_BYTES + HIT_OUT_BYTES) + SLAB_BYTES * wc["node_fetches"] +
-                 TRI_BYTES * wc["slab_crossings"] + BOX_BYTES * wc["box_loads"])
     ref_bytes = N_RAYS * (REF_RAY_IN_BYTES + HIT_OUT_BYTES) + NODE_BYTES * visits_closest
     avg_launch_s = statistics.mean(launch_ms) * 1e-3
     achieved = ref_bytes / avg_launch_s / 1e9
@@ -1008,8 +1002,8 @@ def main():
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded)",
         "config": {"workload": WORKLOAD, "triangles": N_TRIS, "rays": N_RAYS, "nmh_levels": nmh.info()[1],
-                   "l2": "inputs larger than L2: 512 MiB of rays streamed per step; the 64 MB of node records "
-                         "stay L2-resident as in any traversal",
+                   "l2": "inputs larger than L2: 512 MiB of rays streamed per step; the 17 MB of treelet records "
+                         "and 64 MB of node records stay L2-resident as in any traversal",
                    "parallelism": "replicas" if world > 1 else "single GPU"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "traffic_source": traffic_source,
@@ -1023,11 +1017,11 @@ def main():
                      "reference_node_visits_per_ray": visits_closest / N_RAYS,
                      "dram_GBps": traffic / avg_launch_s / 1e9 if traffic else None,
                      "dram_frac": traffic / avg_launch_s / 1e9 / peak if traffic else None,
-                     "limiter": "instruction issue and the L1 data pipe, not DRAM (see the ncu summary): the 64 MB "
-                                "of node records stay in the 129 MB L2, so the algorithmic bytes are served by "
-                                "L1/L2 and their rate can exceed the HBM copy peak",
-                     "traversal_reads_bytes_per_launch": own_bytes,
-                     "traversal_reads_GBps": own_bytes / avg_launch_s / 1e9,
+                     "limiter": "instruction issue, the integer pipe and the L1 data pipe, not DRAM (see the ncu "
+                                "summary): the records (17 MB of treelets, 64 MB of nodes) stay in the 129 MB L2, "
+                                "so the algorithmic bytes are served by L1/L2 and their rate can exceed the HBM "
+                                "copy peak",
+                     "counted_walk": "node by node with box pruning; the timed traversal takes two levels a step",
                      "node_fetches_per_ray": wc["node_fetches"] / N_RAYS,
                      "slab_crossings_per_ray": wc["slab_crossings"] / N_RAYS},
         "e2e": {"value": e2e_value, "unit": "Mrays/s", "h2d_bytes_per_step": N_RAYS * 32,

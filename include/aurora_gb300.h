@@ -349,10 +349,11 @@ aur_status aur_trace_count_visits(aur_ctx* ctx, const aur_nmh* nmh, const aur_ra
 
 /* Test hook: the number of 32-ray chunks that the last aur_trace_closest /
  * aur_trace_any on this context left to the one-ray-per-thread kernel
- * (directions of more than one octant). Synchronizes the context's stream. */
+ * (directions of more than one octant, or origins too far apart). Synchronizes the context's stream. */
 aur_status aur_debug_trace_deferred(aur_ctx* ctx, uint32_t* chunks);
 
-/* Work of this library's traversal (with subtree-box pruning) over n rays:
+/* Work of the node-by-node traversal with subtree-box pruning (the counting
+ * kernels; a trace takes two levels a step and fetches less) over n rays:
  * node records fetched (16-byte slab load), slabs crossed (two triangles,
  * 64 bytes, tested) and children's boxes loaded (48 bytes). No reference
  * counterpart; used for roofline accounting. */
