@@ -611,38 +611,36 @@ __device__ __forceinline__ f3 direct_light(const SceneView& sc, const aur_shader
     for (uint32_t i = 0; i < sc.num_lights; ++i) {
         const aur_light& L = sc.lights[i];
         if (L.type == AUR_LIGHT_AMBIENT) Li = Li + bsdf_f(b) * ((from(L.color) * L.intensity) * L.ambient);
-        if (L.type != AUR_LIGHT_AREA) {
-            // estimateDirectRadianceDelta (radiance.cuh:18-33): no offset
+        // estimateDirectRadiance (radiance.cuh:35-80), light-sampling half, and
+        // estimateDirectRadianceDelta (radiance.cuh:18-33): one sample, no
+        // offset. Both through one shadow trace: its code is most of a kernel
+        // that waits for instructions (4130-triangle sphere in a box, 256x256, 16
+        // samples: 2.95 ms with a trace for each kind, 2.71 with one; the adjoint,
+        // whose sums stay in registers across it, gained nothing: 4.35 to 4.45).
+        const bool area = L.type == AUR_LIGHT_AREA;
+        const int32_t samples = area ? L.samples : 1;
+        f3 acc = mk3(0.0f);
+        for (int32_t j = 0; j < samples; ++j) {
             f3 wdir; float wt, pdf;
-            const f3 Ls = sample_light(L, position, seed, scene, pixel, sample, rix, 0u, wdir, wt, pdf);
-            if (pdf > 0.0f && !zero(Ls)) {
-                const f3 f = bsdf_f(b);
-                if (!zero(f) &&
-                    !occluded(sc, trav, position, wdir, wt))
-                    Li = Li + f * Ls * fmaxf(0.0f, dot(wdir, b.N));
-            }
-        } else {
-            // estimateDirectRadiance (radiance.cuh:35-80), light-sampling half
-            f3 acc = mk3(0.0f);
-            for (int32_t j = 0; j < L.samples; ++j) {
-                f3 Ls = mk3(0.0f);
-                f3 wdir; float wt, lpdf;
-                const f3 Lr = sample_light(L, position, seed, scene, pixel, sample, rix, light_slot(i, (uint32_t)j),
-                                           wdir, wt, lpdf);
-                // Ray::offset(Epsilon) (ray.cuh:184-191)
-                f3 wpos = position;
+            const f3 Ls = sample_light(L, position, seed, scene, pixel, sample, rix,
+                                       area ? light_slot(i, (uint32_t)j) : 0u, wdir, wt, pdf);
+            f3 wpos = position;
+            if (area) {   // Ray::offset(Epsilon) (ray.cuh:184-191)
                 wpos.x += kEpsilon * wdir.x;
                 wpos.y += kEpsilon * wdir.y;
                 wpos.z += kEpsilon * wdir.z;
                 wt += kEpsilon;
-                if (lpdf > 0.0f && !zero(Lr)) {
-                    const f3 f = bsdf_f(b);
-                        if (!zero(f) &&
-                        !occluded(sc, trav, wpos, wdir, wt))
-                        Ls = Ls + f * Lr * fmaxf(0.0f, dot(wdir, b.N));
-                }
-                acc = acc + Ls;
             }
+            if (pdf > 0.0f && !zero(Ls)) {
+                const f3 f = bsdf_f(b);
+                if (!zero(f) && !occluded(sc, trav, wpos, wdir, wt)) {
+                    const f3 c = f * Ls * fmaxf(0.0f, dot(wdir, b.N));
+                    if (area) acc = acc + c;
+                    else Li = Li + c;
+                }
+            }
+        }
+        if (area) {
             const float ns = (float)L.samples;
             Li = Li + mk3(acc.x / ns, acc.y / ns, acc.z / ns);
         }
