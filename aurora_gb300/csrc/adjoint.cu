@@ -44,12 +44,14 @@ namespace {
 constexpr int kAdjThreads = 128;
 // Resident blocks per SM that the replay kernel is compiled for: its lanes
 // diverge and it waits on latency and instruction fetch, so more warps pay for
-// the spills. With per-warp sums (256x256, 16 samples of a 4130-triangle box
-// with a shader each): 4.75 ms at 6 blocks, 4.49 at 8, 4.33 at 10, 4.35 at 12,
-// 4.42 at 14, in the MIS mode 3.49, 3.41, 3.11, 2.99 and 2.88 (8 samples). With
-// a thread's own sums (100k-triangle spheres, 8 samples): 2.13 ms at 8, 2.14 at
-// 10, 2.25 at 12, 2.53 at 14.
-constexpr int adj_blocks(bool few) { return few ? 10 : 12; }
+// the spills. Without a ray stack (replay_diffuse), 256x256: per-warp sums, 16
+// samples of a 4130-triangle box with a shader each: 3.80 ms at 8 blocks, 3.65
+// at 10, 3.73 at 12, 3.97 at 14, in the MIS mode (8 samples) 2.81, 2.70, 2.69
+// and 2.58; a thread's own sums, the 34-triangle box (8 samples): 0.64 ms at 8,
+// 0.65 at 9, 0.66 at 10, 0.67 at 12. With the stack: 4.49 ms at 8, 4.33 at 10,
+// 4.35 at 12, 4.42 at 14, in the MIS mode 3.41, 3.11, 2.99 and 2.88; own sums
+// (100k-triangle spheres) 2.13 at 8, 2.14 at 10, 2.25 at 12.
+constexpr int adj_blocks(bool generic, bool few) { return generic ? (few ? 10 : 12) : (few ? 8 : 10); }
 constexpr uint32_t kSharedLights = 64;
 
 // Per-unit-colour radiance of a light sample (Lr = color * s), light.cuh:228-259.
@@ -320,9 +322,71 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
     while (nm > 0) close(mk[--nm]);
 }
 
-// Replay kernel: one thread per camera sample of samples [s0, s0 + nb). kFew: at most kFewShaders shaders.
-template <bool kMis, bool kTiny, bool kFew>
-__global__ void __launch_bounds__(kAdjThreads, adj_blocks(kFew)) k_adj_replay(SceneView sc, aur_camera cam,
+// The same replay for scenes without specular shaders: one ray in flight per
+// sample, no ray stack, and every subtree is the rest of the path, so all of
+// them end where the path does. Same operations in the same order as
+// replay_stack(). What bounds the replay is instruction fetch and the local
+// memory of its stack: without stack, reflection and refraction the box of
+// adj_blocks takes 3.65 ms (4.35 with them), the 34-triangle box 0.64 (0.86).
+template <bool kMis, typename Trav, typename Grads>
+__device__ __forceinline__ void replay_diffuse(const SceneView& sc, uint32_t max_depth, uint32_t mode, uint32_t seed,
+                                               uint32_t scene, uint32_t pixel, uint32_t sample, const PathRay& primary,
+                                               const Trav& trav, const f3& g, Grads& grads,
+                                               float* __restrict__ d_light, f3& gl0, uint32_t* err) {
+    struct Marker {
+        f3 col0, c1;          // colour before the subtree, the bouncing vertex's Lambert colour
+        uint32_t si;
+    };
+    Marker mk[AUR_MAX_DEPTH];
+    uint32_t nm = 0;          // bounces, also the depth
+    f3 pos = primary.pos, dir = primary.dir, thr = primary.thr, col = mk3(0.0f);
+    float prev_pdf = 0.0f;
+    const bool path = kMis || mode == AUR_MODE_PATH;
+    for (;;) {
+        float t = kInfinity, u = 0.0f, v = 0.0f;
+        const uint32_t tri = closest_hit(sc, trav, pos, dir, t, u, v);
+        if (tri == kNoPrim) break;
+        const f3 position = pos + (dir * t);
+        const f3 wo = -dir;
+        const uint32_t sid = sc.sids[tri];
+        const uint32_t si = sid > 0 ? sid - 1 : 0;
+        const aur_shader* sh = sc.shaders + si;
+        const Bsdf b = get_bsdf(sc, sh, tri, u, v);
+        const f3 f = bsdf_f(b);
+        const float ew = kMis ? emission_weight(sc, tri, dir, t, prev_pdf) : 1.0f;
+        f3 Dp;
+        const f3 Li = direct_grad<kMis>(sc, sh, b, f, position, wo, ew, nm + 1 <= max_depth, seed, scene, pixel, sample,
+                                        nm, thr, g, d_light, gl0, Dp, grads, si, trav, err);
+        grads.add_diffuse(si, sh, g * (thr * Dp));
+        col = col + Li * thr;
+        if (!path || nm + 1 > max_depth) break;
+        f3 wi, nthr;
+        if (!(kMis ? mis_bounce(b, wo, thr, seed, scene, pixel, sample, nm, wi, nthr, prev_pdf)
+                   : diffuse_bounce(b, wo, thr, seed, scene, pixel, sample, nm, wi, nthr, prev_pdf)))
+            break;
+        mk[nm].col0 = col;
+        mk[nm].c1 = b.color1;
+        mk[nm].si = si;
+        ++nm;
+        pos = position;
+        dir = wi;
+        thr = nthr;
+    }
+    while (nm > 0) {
+        const Marker m = mk[--nm];
+        const f3 sub = col - m.col0;
+        f3 dc;
+        dc.x = m.c1.x != 0.0f ? sub.x / m.c1.x : 0.0f;
+        dc.y = m.c1.y != 0.0f ? sub.y / m.c1.y : 0.0f;
+        dc.z = m.c1.z != 0.0f ? sub.z / m.c1.z : 0.0f;
+        grads.add_diffuse(m.si, sc.shaders + m.si, g * dc);
+    }
+}
+
+// Replay kernel: one thread per camera sample of samples [s0, s0 + nb). kGeneric: the scene has specular shaders;
+// kFew: at most kFewShaders shaders.
+template <bool kGeneric, bool kMis, bool kTiny, bool kFew>
+__global__ void __launch_bounds__(kAdjThreads, adj_blocks(kGeneric, kFew)) k_adj_replay(SceneView sc, aur_camera cam,
                                                                             aur_render_params p, uint32_t s0,
                                                                             uint32_t nb,
                                                                             const float4* __restrict__ d_image,
@@ -352,8 +416,11 @@ __global__ void __launch_bounds__(kAdjThreads, adj_blocks(kFew)) k_adj_replay(Sc
         const float4 di = d_image[pix];
         const float w = 1.0f / (float)p.spp;
         const f3 g = mk3(di.x * w, di.y * w, di.z * w);
-        replay_stack<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, grads,
-                           shared_lights ? s_light : d_light, gl0, err);
+        float* dl = shared_lights ? s_light : d_light;
+        if constexpr (kGeneric)
+            replay_stack<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, grads, dl, gl0, err);
+        else
+            replay_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, grads, dl, gl0, err);
     }
     if constexpr (kFew) {      // the block's sums, one atomic per entry
         __shared__ float s_sum[kAdjThreads / 32][6 * kFewShaders];
@@ -431,17 +498,14 @@ aur_status aur_render_adjoint(aur_ctx* ctx, const aur_scene* scene, const aur_ca
     for (uint32_t s = s0; s < s1; s += batch) {
         const uint32_t nb = std::min(batch, s1 - s);
         const uint32_t grid = cdiv(P * nb, kAdjThreads);
-        auto go = [&](auto m, auto tiny, auto few) {
-            k_adj_replay<m.value, tiny.value, few.value><<<grid, kAdjThreads, 0, ctx->stream>>>(
+        auto go = [&](auto spec, auto m, auto tiny, auto few) {
+            k_adj_replay<spec.value, m.value, tiny.value, few.value><<<grid, kAdjThreads, 0, ctx->stream>>>(
                 sv, *camera, p, s, nb, di, d_diffuse, d_light_color, d_emission, scene->num_shaders, ctx->d_flags);
         };
-        auto pick = [&](auto m, auto tiny) {
-            if (scene->num_shaders <= kFewShaders) go(m, tiny, std::true_type{});
-            else go(m, tiny, std::false_type{});
-        };
-        const bool tiny = scene->nmh->count <= kTinyTris;
-        if (mis) tiny ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
-        else tiny ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{});
+        launch_variant(scene, mis, [&](auto spec, auto m, auto tiny) {
+            if (scene->num_shaders <= kFewShaders) go(spec, m, tiny, std::true_type{});
+            else go(spec, m, tiny, std::false_type{});
+        });
     }
     AUR_CUDA(cudaGetLastError());
     return AUR_OK;

@@ -9,6 +9,8 @@
 // bounce of BSDF::samplef (bsdf.cuh:222-236) with an RGB throughput.
 #pragma once
 
+#include <type_traits>
+
 #include "aur_math.cuh"
 #include "aur_traverse.cuh"
 #include "aur_wide.cuh"
@@ -855,6 +857,23 @@ __device__ __forceinline__ PathRay camera_ray(const aur_camera& cam, uint32_t W,
     r.pdf = 0.0f;
     r.dir = normalize(px * from(cam.right) * cam.tanfov_x + py * from(cam.up) * cam.tanfov_y + from(cam.forward));
     return r;
+}
+
+// Calls f with the scene's kernel variant: specular materials (the integrator
+// and replay with the ray stack), the MIS estimator, few triangles.
+template <typename F>
+void launch_variant(const aur_scene* scene, bool mis, F f) {
+    auto pick = [&](auto spec, auto m) {
+        if (scene->nmh->count <= kTinyTris) f(spec, m, std::true_type{});
+        else f(spec, m, std::false_type{});
+    };
+    if (scene->has_specular) {
+        if (mis) pick(std::true_type{}, std::true_type{});
+        else pick(std::true_type{}, std::false_type{});
+    } else {
+        if (mis) pick(std::false_type{}, std::true_type{});
+        else pick(std::false_type{}, std::false_type{});
+    }
 }
 
 }  // namespace aur

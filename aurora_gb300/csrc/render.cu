@@ -235,27 +235,6 @@ aur_status check_params(const aur_render_params* p) {
 
 using namespace aur;
 
-namespace {
-
-// Calls f with the scene's kernel variant: specular materials (the integrator
-// with the ray stack), the MIS estimator, few triangles.
-template <typename F>
-void launch_variant(const aur_scene* scene, bool mis, F f) {
-    auto pick = [&](auto spec, auto m) {
-        if (scene->nmh->count <= kTinyTris) f(spec, m, std::true_type{});
-        else f(spec, m, std::false_type{});
-    };
-    if (scene->has_specular) {
-        if (mis) pick(std::true_type{}, std::true_type{});
-        else pick(std::true_type{}, std::false_type{});
-    } else {
-        if (mis) pick(std::false_type{}, std::true_type{});
-        else pick(std::false_type{}, std::false_type{});
-    }
-}
-
-}  // namespace
-
 extern "C" {
 
 aur_status aur_render(aur_ctx* ctx, const aur_scene* scene, const aur_camera* camera, const aur_render_params* params,
