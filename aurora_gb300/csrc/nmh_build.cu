@@ -109,11 +109,21 @@ __host__ __device__ __forceinline__ uint64_t left_base(uint64_t k, uint64_t L0, 
 // i >= count_in is the even-padding duplicate of the last triangle.
 // A coordinate that is NaN or infinite sets bit 8 of *err: the reference's
 // float sorts have no defined order for NaN, so the build refuses such soups.
+// Thread k also writes node k's layout: segment start, left-child triangle
+// count and left base (a launch of its own before).
 __global__ void k_bounds(const float* __restrict__ V, uint32_t N, size_t S, uint32_t count_in,
                          float* __restrict__ mn, float* __restrict__ mx, uint32_t* __restrict__ keys,
-                         uint32_t* __restrict__ vals, uint32_t* __restrict__ err) {
+                         uint32_t* __restrict__ vals, uint32_t* __restrict__ nstart, uint32_t* __restrict__ nnuml,
+                         uint32_t* __restrict__ nlbase, uint32_t* __restrict__ err) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
+    const uint32_t n = N / 2;
+    if (i < n) {
+        const uint32_t L0 = (1u << level_of(i)) - 1u;
+        nstart[i] = (uint32_t)segment_start(i, L0, n);
+        nnuml[i] = (2u * i + 1u < n) ? (uint32_t)(2 * subtree_nodes(2u * i + 1u, n)) : 0u;
+        nlbase[i] = (uint32_t)left_base(i, L0, n);
+    }
     const uint32_t src = i < count_in ? i : count_in - 1;
     const float* v = V + (size_t)src * 9;
     float c[9];
@@ -135,7 +145,16 @@ __global__ void k_bounds(const float* __restrict__ V, uint32_t N, size_t S, uint
     }
 }
 
-// Radix sort, pass histogram: hist[(axis*256 + digit) * nb + block].
+// Sorts of at most this many tiles (65,536 keys) leave out the scan launch of
+// each pass: the scatter's blocks add up the tiles' counts themselves. (20k
+// triangles 0.333 -> 0.314 ms a build, 3k 0.233 -> 0.218, 60k 0.352 -> 0.349;
+// at 120k and 250k, with 64 and 122 tiles, the sums cost 0.01 and 0.03 ms more
+// than the launches.)
+constexpr uint32_t kFewTiles = 32;
+
+// Radix sort, pass histogram: hist[(axis*256 + digit) * nb + block], with kFew
+// hist[(axis*nb + block) * 256 + digit].
+template <bool kFew>
 __global__ void k_radix_hist(const uint32_t* __restrict__ keys, uint32_t N, size_t S, int shift,
                              uint32_t* __restrict__ hist, uint32_t nb) {
     __shared__ uint32_t h[256];
@@ -150,7 +169,8 @@ __global__ void k_radix_hist(const uint32_t* __restrict__ keys, uint32_t N, size
         if (idx < N) atomicAdd(&h[(k[idx] >> shift) & 255u], 1u);
     }
     __syncthreads();
-    hist[((size_t)axis * 256 + threadIdx.x) * nb + blockIdx.x] = h[threadIdx.x];
+    if (kFew) hist[((size_t)axis * nb + blockIdx.x) * 256 + threadIdx.x] = h[threadIdx.x];
+    else hist[((size_t)axis * 256 + threadIdx.x) * nb + blockIdx.x] = h[threadIdx.x];
 }
 
 // Block-wide exclusive scan of one value per thread (blockDim.x <= 1024).
@@ -203,6 +223,9 @@ __global__ void k_radix_scan_rows(uint32_t* __restrict__ hist, uint32_t nb, uint
 // sorted in shared memory and written out in digit runs, so that neighbouring
 // threads store neighbouring words. (3 x 1M keys with a cold L2: 28 us a
 // pass; a barrier-separated round per 256 keys with scattered stores took 41.)
+// kFew: hist holds the counts of the tiles (k_radix_hist<true>), not their
+// scan (k_radix_scan_rows), and totals is not read.
+template <bool kFew>
 __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* __restrict__ kin,
                                                             const uint32_t* __restrict__ vin,
                                                             uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
@@ -258,9 +281,20 @@ __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* __re
         }
         uint32_t tot;
         const uint32_t start = block_exclusive_scan(run, s_warp, tot);
-        const uint32_t out = block_exclusive_scan(totals[axis * 256 + t], s_warp, tot);
+        uint32_t before = 0, all = 0;      // the digit's keys in earlier tiles, in all
+        if (kFew) {
+            for (uint32_t b = 0; b < nb; ++b) {
+                const uint32_t c = hist[((size_t)axis * nb + b) * 256 + t];
+                if (b < blockIdx.x) before += c;
+                all += c;
+            }
+        } else {
+            before = hist[((size_t)axis * 256 + t) * nb + blockIdx.x];
+            all = totals[axis * 256 + t];
+        }
+        const uint32_t out = block_exclusive_scan(all, s_warp, tot);
         s_start[t] = start;
-        s_out[t] = out + hist[((size_t)axis * 256 + t) * nb + blockIdx.x] - start;
+        s_out[t] = out + before - start;
     }
     __syncthreads();
 #pragma unroll
@@ -284,18 +318,6 @@ __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* __re
             atomicOr(err, 4u);
         }
     }
-}
-
-// Per-node layout table: segment start, left-child triangle count and
-// left base, for every node of the heap.
-__global__ void k_node_table(uint32_t n, uint32_t* __restrict__ nstart, uint32_t* __restrict__ nnuml,
-                             uint32_t* __restrict__ nlbase) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t L0 = (1u << level_of(k)) - 1u;
-    nstart[k] = (uint32_t)segment_start(k, L0, n);
-    nnuml[k] = (2u * k + 1u < n) ? (uint32_t)(2 * subtree_nodes(2u * k + 1u, n)) : 0u;
-    nlbase[k] = (uint32_t)left_base(k, L0, n);
 }
 
 // Bit 16 of the error word: a look-back wait gave up. The lists of that
@@ -719,7 +741,7 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_finish(const uint32_t* 
         const uint64_t avail = (uint64_t)n - G0;
         const uint32_t nd = (uint32_t)((1ull << d) < avail ? (1ull << d) : avail);
         const uint32_t a = lv % 3u, b = (lv + 1) % 3u, c = (lv + 2) % 3u;
-        // the depth's part of the node table (k_node_table), relative to this block's first node
+        // the depth's part of the node table (k_bounds), relative to this block's first node
         {
             const uint32_t o0 = nstart[G0], l0 = nlbase[G0];
             for (uint32_t r = t; r < nd; r += kLocalThreads) {
@@ -1334,7 +1356,8 @@ void enqueue_build(Seq& q, const BuildArgs& b) {
     const uint32_t ntiles = cdiv(N, kTile);
 
     q.memset(base + L.zero, L.zero_end - L.zero);
-    q.launch(k_bounds, dim3(cdiv(N, 256)), dim3(256), 0, b.V, N, S, b.count, mn, mx, keys, vals, b.flags);
+    q.launch(k_bounds, dim3(cdiv(N, 256)), dim3(256), 0, b.V, N, S, b.count, mn, mx, keys, vals, ns, nl,
+             nlb, b.flags);
     // three stable LSD radix sorts of (min-key, prim id); result in keys/vals
     for (int pass = 0; pass < 4; ++pass) {
         const int shift = pass * 8;
@@ -1342,15 +1365,20 @@ void enqueue_build(Seq& q, const BuildArgs& b) {
         uint32_t* vin = (pass & 1) ? v2 : vals;
         uint32_t* kout = (pass & 1) ? keys : k2;
         uint32_t* vout = (pass & 1) ? vals : v2;
-        q.launch(k_radix_hist, dim3(nb, 3), dim3(kThreads), 0, kin, N, S, shift, hist, nb);
-        q.launch(k_radix_scan_rows, dim3(256, 3), dim3(1024), 0, hist, nb, tot);
-        q.launch(k_radix_scatter, dim3(nb, 3), dim3(kThreads), 0, kin, vin, kout, vout, N, S, shift, hist, tot, nb,
-                 b.flags);
+        if (nb <= kFewTiles) {
+            q.launch(k_radix_hist<true>, dim3(nb, 3), dim3(kThreads), 0, kin, N, S, shift, hist, nb);
+            q.launch(k_radix_scatter<true>, dim3(nb, 3), dim3(kThreads), 0, kin, vin, kout, vout, N, S, shift, hist, tot,
+                     nb, b.flags);
+        } else {
+            q.launch(k_radix_hist<false>, dim3(nb, 3), dim3(kThreads), 0, kin, N, S, shift, hist, nb);
+            q.launch(k_radix_scan_rows, dim3(256, 3), dim3(1024), 0, hist, nb, tot);
+            q.launch(k_radix_scatter<false>, dim3(nb, 3), dim3(kThreads), 0, kin, vin, kout, vout, N, S, shift, hist,
+                     tot, nb, b.flags);
+        }
     }
     // lists: vals = sorted pids per axis (buffer A), v2 = buffer B
     uint32_t* listA = vals;
     uint32_t* listB = v2;
-    q.launch(k_node_table, dim3(cdiv(n, 256)), dim3(256), 0, n, ns, nl, nlb);
 
     // levels above lv0 over the whole soup, the rest per subtree in shared memory
     const uint32_t lv0 = local_level(n, levels);
