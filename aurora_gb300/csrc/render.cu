@@ -21,10 +21,11 @@ namespace {
 
 constexpr int kRenderThreads = 128;
 // Resident blocks per SM that the fused sample kernel is compiled for,
-// measured among 4 to 16. Trees: path mode 1.88 ms at 8, 1.91 at 6 and 10, 1.94
-// at 14 (200k-triangle spheres); the MIS estimator 2.41 at 6 to 8, 2.35 at 14
+// measured among 4 to 16. Trees: path mode 1.74 ms at 6 and 7, 1.75 at 8, 1.77 at
+// 9, 1.82 at 10 (200k-triangle spheres), 13.1, 13.7, 13.0, 13.2 and 14.0 ms (200k-
+// triangle terrain); the MIS estimator 2.41 ms at 6 to 8, 2.35 at 14
 // (4130-triangle box; its lanes diverge, and more warps to switch between pay
-// for the spills). Tiny scenes: 0.86 ms at 6 and 7, 0.88 at 5 and 8, 0.92 at 14
+// for the spills). Tiny scenes: 0.85 ms at 5, 6 and 8, 0.87 at 7, 0.88 at 9
 // (256x256 box, 16 samples); the MIS estimator 1.14 at 5 and 7, 1.18 at 8 and
 // 14 (301x233 emissive box, 9 samples). The per-tile kernel (k_raytrace_mc)
 // runs grids of one 65,536-ray tile, too small for occupancy to matter, and is
