@@ -282,25 +282,35 @@ __device__ __forceinline__ uint32_t wide_boxes(uint32_t acc, uint32_t xn, uint32
 
 // ------------------------------------------------------------ ray and state
 struct WideRay {
-    f3 pos, dir, inv;     // inv: reciprocal direction, components clamped to +-1e20
+    f3 pos, dir, inv;     // inv: reciprocal direction, clamped (wide_ray)
     uint32_t order;       // bit 31 - b: the ray visits the second child first on level b (0 < b < 31)
 };
 
-__device__ __forceinline__ float wide_recip(float d) { return 1.0f / copysignf(fmaxf(fabsf(d), 1e-20f), d); }
+__device__ __forceinline__ float wide_recip(float d, float least) {
+    return 1.0f / copysignf(fmaxf(fabsf(d), least), d);
+}
 
 __device__ __forceinline__ uint32_t wide_order(bool nx, bool ny, bool nz) {
     return (nx ? 0x12492492u : 0u) | (ny ? 0x49249249u : 0u) | (nz ? 0x24924924u : 0u);
 }
 
+// Components below 1e-20, and below 1e-12 of the largest, are taken as that
+// for the box tests. Over the distance to a hit the ray is moved sideways by at
+// most 1e-12 of that distance, far below the boxes' padding, and the
+// reciprocals of axis-parallel rays stay finite.
 __device__ __forceinline__ void wide_ray(WideRay& r, const f3& pos, const f3& dir) {
     r.pos = pos;
     r.dir = dir;
-    r.inv = mk3(wide_recip(dir.x), wide_recip(dir.y), wide_recip(dir.z));
+    const float least = fminf(1e-20f, 1e-12f * fmaxf(longest(dir), kShortDir));
+    r.inv = mk3(wide_recip(dir.x, least), wide_recip(dir.y, least), wide_recip(dir.z, least));
     r.order = wide_order(dir.x < 0.0f, dir.y < 0.0f, dir.z < 0.0f);
 }
 
-// What a ray has found: best is the NMH position of the triangle, t2 the
-// smallest t of any other triangle it meets (tmax at the start).
+// What a ray has found: best is the NMH position of the triangle (kNoPrim:
+// none; kWalkRay: the ray is too short for box tests, the checks walk it), t2
+// the smallest t of any other triangle it meets (tmax at the start).
+constexpr uint32_t kWalkRay = 0xFFFFFFFEu;
+
 struct WideHit {
     float t, t2;
     uint32_t best;
@@ -327,8 +337,10 @@ __device__ __forceinline__ void wide_init(WideState& s, uint32_t levels) {
     s.at_pair = false;
 }
 
-// Starts a ray. Returns false when it can hit nothing: no t in (Epsilon, tmax),
-// or a component that is NaN or infinite (every t test of such a ray fails).
+// Starts a ray. Returns false when there is nothing to traverse: it can hit
+// nothing (no t in (Epsilon, tmax), no direction, or a component that is NaN or
+// infinite: every t test of such a ray fails), or its direction is short and
+// the exact walk takes it (h.best is kWalkRay).
 __device__ __forceinline__ bool wide_begin(WideRay& r, WideState& s, WideHit& h, const WideView& w, const f3& pos,
                                            const f3& dir, float tmax) {
     wide_ray(r, pos, dir);
@@ -336,7 +348,11 @@ __device__ __forceinline__ bool wide_begin(WideRay& r, WideState& s, WideHit& h,
     h.t = h.t2 = tmax;
     h.best = kNoPrim;
     const float z = ((pos.x * 0.0f + pos.y * 0.0f) + (pos.z * 0.0f + dir.x * 0.0f)) + (dir.y * 0.0f + dir.z * 0.0f);
-    return w.nodes != 0u && tmax > kEpsilon && z == 0.0f;
+    if (!(w.nodes != 0u && tmax > kEpsilon && z == 0.0f)) return false;
+    const float len = longest(dir);
+    if (len >= kShortDir) return true;
+    if (len > 0.0f) h.best = kWalkRay;
+    return false;
 }
 
 // Tests the ten boxes of the current treelet against (0, lim]: its pending
@@ -507,13 +523,15 @@ struct WideQueue {
 
 constexpr unsigned long long kNoKey = ~0ull;
 
+// best: WideHit::best as wide_begin left it.
 template <WideMode kMode>
-__device__ __forceinline__ void queue_ray(WideQueue& q, uint32_t lane, const f3& pos, const f3& dir, float tmax) {
+__device__ __forceinline__ void queue_ray(WideQueue& q, uint32_t lane, const f3& pos, const f3& dir, float tmax,
+                                          uint32_t best) {
     q.pd[lane] = make_float4(pos.x, pos.y, pos.z, dir.x);
     q.d[lane] = make_float2(dir.y, dir.z);
     // a triangle at exactly tmax is not a hit: no (tmax, prim id) is below (tmax, 0)
     q.key[lane] = kMode == kWideClosest ? (unsigned long long)__float_as_uint(tmax) << 32 : kNoKey;
-    q.best[lane] = kNoPrim;
+    q.best[lane] = best;
     q.t2[lane] = __float_as_uint(tmax);
 }
 
@@ -585,7 +603,7 @@ __device__ __forceinline__ void wide_warp(const WideView& w, WideQueue& q, bool 
     WideState s;
     bool running = wide_begin(r, s, h, w, pos, dir, tmax) && valid;
     __syncwarp();
-    queue_ray<kMode>(q, lane, pos, dir, tmax);
+    queue_ray<kMode>(q, lane, pos, dir, tmax, h.best);
     __syncwarp();
     float lim = tmax;
     uint32_t count = 0, seq = 0;
@@ -696,8 +714,10 @@ static inline unsigned long long fma2(unsigned long long a, unsigned long long b
 // Bit j: triangle j is kept.
 __device__ __forceinline__ uint64_t tiny_filter(const TinyStage& s, uint32_t count, const f3& pos, const f3& dir) {
     const uint64_t all = count >= 64u ? ~0ull : (1ull << count) - 1ull;
-    const float scale = 4.0e-6f * (sqrtf(dot(pos, pos)) + __uint_as_float(s.radius)) * sqrtf(dot(dir, dir));
-    if (!(scale < 1.0e24f)) return all;
+    const float dd = dot(dir, dir);
+    const float scale = 4.0e-6f * (sqrtf(dot(pos, pos)) + __uint_as_float(s.radius)) * sqrtf(dd);
+    // products beyond the float range, or a length that its square's underflow makes too small
+    if (!(scale < 1.0e24f && dd > 1.0e-30f)) return all;
     const f3 m = cross(pos, dir);
     const unsigned long long dx = pack2(dir.x, dir.x), dy = pack2(dir.y, dir.y), dz = pack2(dir.z, dir.z);
     const unsigned long long mx = pack2(m.x, m.x), my = pack2(m.y, m.y), mz = pack2(m.z, m.z);
@@ -803,7 +823,8 @@ static __device__ __noinline__ float2 path_range(const float4* recs, uint32_t tr
 }
 
 // The walk of intersect() itself, for a ray whose triangle fails the check
-// (its slab ranges exclude the triangle by rounding): (t, u, v, NMH position).
+// (its slab ranges exclude the triangle by rounding), or whose direction is
+// short: (t, u, v, NMH position).
 template <bool kAny>
 static __device__ __forceinline__ float4 exact_walk(const float4* recs, uint32_t nodes, const uint32_t* perm, float px, float py,
                                           float pz, float dx, float dy, float dz, float tmax) {
@@ -845,19 +866,21 @@ __device__ __forceinline__ void finish_closest(const WideView& w, const WideRay&
                                                float& v) {
     u = v = 0.0f;
     if (h.best == kNoPrim) return;
-    float q[9];
-    const float* src = w.verts + (size_t)h.best * 9;
+    if (h.best != kWalkRay) {
+        float q[9];
+        const float* src = w.verts + (size_t)h.best * 9;
 #pragma unroll
-    for (int j = 0; j < 9; ++j) q[j] = __ldg(src + j);
-    float t, E, X;
-    intersect_tri(r.pos, r.dir, mk3(q[0], q[3], q[6]), mk3(q[1] - q[0], q[4] - q[3], q[7] - q[6]),
-                  mk3(q[2] - q[0], q[5] - q[3], q[8] - q[6]), u, v, t);
-    own_range(q, r.pos, r.dir, E, X);
-    // a zero direction component has 0/0 distances: only the path's own slabs tell
-    const bool quick = r.dir.x != 0.0f && r.dir.y != 0.0f && r.dir.z != 0.0f && E <= X && visited_before(E, h);
-    if (quick) return;
-    const float2 range = path_range(w.recs, h.best, r.pos.x, r.pos.y, r.pos.z, r.dir.x, r.dir.y, r.dir.z);
-    if (range.x <= range.y && visited_before(range.x, h)) return;
+        for (int j = 0; j < 9; ++j) q[j] = __ldg(src + j);
+        float t, E, X;
+        intersect_tri(r.pos, r.dir, mk3(q[0], q[3], q[6]), mk3(q[1] - q[0], q[4] - q[3], q[7] - q[6]),
+                      mk3(q[2] - q[0], q[5] - q[3], q[8] - q[6]), u, v, t);
+        own_range(q, r.pos, r.dir, E, X);
+        // a zero direction component has 0/0 distances: only the path's own slabs tell
+        const bool quick = r.dir.x != 0.0f && r.dir.y != 0.0f && r.dir.z != 0.0f && E <= X && visited_before(E, h);
+        if (quick) return;
+        const float2 range = path_range(w.recs, h.best, r.pos.x, r.pos.y, r.pos.z, r.dir.x, r.dir.y, r.dir.z);
+        if (range.x <= range.y && visited_before(range.x, h)) return;
+    }
     const float4 e = exact_walk<false>(w.recs, w.nodes, w.perm, r.pos.x, r.pos.y, r.pos.z, r.dir.x, r.dir.y, r.dir.z, tmax);
     h.t = e.x;
     u = e.y;
@@ -870,15 +893,17 @@ __device__ __forceinline__ void finish_closest(const WideView& w, const WideRay&
 // intersectAny() finds.
 __device__ __forceinline__ uint32_t finish_any(const WideView& w, const WideRay& r, uint32_t best, float tmax) {
     if (best == kNoPrim) return best;
-    float q[9];
-    const float* src = w.verts + (size_t)best * 9;
+    if (best != kWalkRay) {
+        float q[9];
+        const float* src = w.verts + (size_t)best * 9;
 #pragma unroll
-    for (int j = 0; j < 9; ++j) q[j] = __ldg(src + j);
-    float E, X;
-    own_range(q, r.pos, r.dir, E, X);
-    if (r.dir.x != 0.0f && r.dir.y != 0.0f && r.dir.z != 0.0f && E <= X && E <= tmax) return best;
-    const float2 range = path_range(w.recs, best, r.pos.x, r.pos.y, r.pos.z, r.dir.x, r.dir.y, r.dir.z);
-    if (range.x <= range.y && range.x <= tmax) return best;
+        for (int j = 0; j < 9; ++j) q[j] = __ldg(src + j);
+        float E, X;
+        own_range(q, r.pos, r.dir, E, X);
+        if (r.dir.x != 0.0f && r.dir.y != 0.0f && r.dir.z != 0.0f && E <= X && E <= tmax) return best;
+        const float2 range = path_range(w.recs, best, r.pos.x, r.pos.y, r.pos.z, r.dir.x, r.dir.y, r.dir.z);
+        if (range.x <= range.y && range.x <= tmax) return best;
+    }
     const float4 e = exact_walk<true>(w.recs, w.nodes, w.perm, r.pos.x, r.pos.y, r.pos.z, r.dir.x, r.dir.y, r.dir.z, tmax);
     return __float_as_uint(e.w);
 }

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_wide(WideView w, con
                     const float4 r1 = rays[2 * (size_t)i + 1];
                     WideHit h;
                     running = wide_begin(r, s, h, w, mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), r0.w);
-                    queue_ray<kMode>(q, lane, r.pos, r.dir, r0.w);
+                    queue_ray<kMode>(q, lane, r.pos, r.dir, r0.w, h.best);
                     lim = r0.w;
                     seq = 0;
                 }

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_extend(WfArgs a) {
                     const float4 o = a.o[slot], d = a.d[slot];
                     WideHit h;
                     running = wide_begin(r, s, h, w, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), kInfinity);
-                    queue_ray<kWideClosest>(q, lane, r.pos, r.dir, kInfinity);
+                    queue_ray<kWideClosest>(q, lane, r.pos, r.dir, kInfinity, h.best);
                     lim = kInfinity;
                 }
             }
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_shadow(WfArgs a) {
                     sw.scene[lane] = scene;
                     WideHit h;
                     running = wide_begin(r, s, h, w, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w);
-                    queue_ray<kWideAny>(q, lane, r.pos, r.dir, o.w);
+                    queue_ray<kWideAny>(q, lane, r.pos, r.dir, o.w, h.best);
                     lim = o.w;
                 }
             }
