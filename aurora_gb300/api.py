@@ -242,8 +242,8 @@ def hits_to_numpy(hits_dev):
 
 
 def trace_deferred(ctx):
-    """Chunks of 32 rays that the context's last device trace left to the
-    one-ray-per-thread kernel (test hook)."""
+    """Mixed chunks of 32 rays in the context's last device trace: those that
+    went one ray per lane (test hook)."""
     c = ctypes.c_uint32()
     check(lib().aur_debug_trace_deferred(ctx.handle, ctypes.byref(c)))
     return c.value

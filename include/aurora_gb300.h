@@ -322,9 +322,10 @@ aur_status aur_generate_tb(aur_ctx* ctx, const float* normals, uint32_t count, f
 /* Closest hit for n rays (intersect(), kernels/lib/intersect.cuh:95-152).
  * rays, hits: device. Ties in t go to the lower original prim id. Rays are
  * taken in chunks of 32 consecutive rays: a chunk whose directions share
- * their octant (signs of x, y, z) is traversed by one warp together, which
- * is fastest for coherent rays (a camera's, rays toward one light); the
- * other chunks are traversed one ray per lane over two-level nodes. Results are the same. The
+ * their octant (signs of x, y, z) and lie close together is traversed by one
+ * warp together, which is fastest for coherent rays (a camera's, rays toward
+ * one light); the other chunks are traversed one ray per lane over two-level
+ * nodes. Results are the same. Directions need not be unit vectors. The
  * first call with more rays than before allocates 4 bytes per 32 rays. */
 aur_status aur_trace_closest(aur_ctx* ctx, const aur_nmh* nmh, const aur_ray* rays, uint32_t n, aur_hit* hits);
 /* Any hit (shadow ray, intersectAny(), intersect.cuh:36-86): occluder[i] is
@@ -348,8 +349,11 @@ aur_status aur_trace_count_visits(aur_ctx* ctx, const aur_nmh* nmh, const aur_ra
                                   unsigned long long node_visits[2]);
 
 /* Test hook: the number of 32-ray chunks that the last aur_trace_closest /
- * aur_trace_any on this context left to the one-ray-per-thread kernel
- * (directions of more than one octant, or origins too far apart). Synchronizes the context's stream. */
+ * aur_trace_any on this context found to be mixed: directions of more than one
+ * octant, or origins too far apart. A launch of more than 768 rays per SM
+ * leaves them to a second kernel, which refills its lanes with further rays; a
+ * smaller one traces them one ray per lane on the spot. 0 for an NMH of at
+ * most 64 triangles. Synchronizes the context's stream. */
 aur_status aur_debug_trace_deferred(aur_ctx* ctx, uint32_t* chunks);
 
 /* Work of the node-by-node traversal with subtree-box pruning (the counting
