@@ -21,6 +21,7 @@ struct SceneView {
     const float4* recs;
     const uint4* wide;
     uint32_t nodes, levels;
+    float reach;               // WideView::reach
     const uint32_t* perm;
     const float* normals;      // NMH order, 9 floats per triangle
     const uint16_t* sids;      // NMH order, 1-based
@@ -68,7 +69,7 @@ __device__ __forceinline__ auto make_trav(const SceneView& sc) {
 }
 
 __device__ __forceinline__ WideView tree_of(const SceneView& sc) {
-    return WideView{sc.recs, sc.wide, sc.perm, sc.verts, sc.nodes, sc.levels};
+    return WideView{sc.recs, sc.wide, sc.perm, sc.verts, sc.nodes, sc.levels, sc.reach};
 }
 
 // Closest hit over (Epsilon, t): the NMH position (kNoPrim: none), t, u, v.

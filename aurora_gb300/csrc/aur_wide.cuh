@@ -60,14 +60,24 @@ struct WideView {
     const float* verts;       // NMH order, 9 floats per triangle
     uint32_t nodes;           // NMH nodes
     uint32_t levels;          // NMH levels
+    // No triangle's det (intersect_tri) exceeds this times the largest
+    // component of the direction: the six products of two edge components and
+    // one of the direction, edges no longer than the soup's extent.
+    float reach = INFINITY;
 
     // the tree that a lane's ray runs in (WideQueue): the same for all
     __device__ __forceinline__ const float4* recs_of(uint32_t) const { return recs; }
     __device__ __forceinline__ const uint32_t* perm_of(uint32_t) const { return perm; }
 };
 
+// WideView::reach of an NMH (infinite where the extent is unknown, and where
+// its square overflows).
+inline float wide_reach(const aur_nmh* nmh) {
+    return nmh->extent > 0.0f ? 6.01f * nmh->extent * nmh->extent : INFINITY;
+}
+
 inline WideView wide_view(const aur_nmh* nmh) {
-    return WideView{nmh->node_recs, nmh->wide, nmh->perm, nmh->verts, nmh->nodes, nmh->levels};
+    return WideView{nmh->node_recs, nmh->wide, nmh->perm, nmh->verts, nmh->nodes, nmh->levels, wide_reach(nmh)};
 }
 
 // Largest origin spread of a warp packet: 1/64 of the soup's extent. Rays
@@ -339,8 +349,9 @@ __device__ __forceinline__ void wide_init(WideState& s, uint32_t levels) {
 
 // Starts a ray. Returns false when there is nothing to traverse: it can hit
 // nothing (no t in (Epsilon, tmax), no direction, or a component that is NaN or
-// infinite: every t test of such a ray fails), or its direction is short and
-// the exact walk takes it (h.best is kWalkRay).
+// infinite: every t test of such a ray fails), or its direction is short. The
+// exact walk takes short ones (h.best is kWalkRay) where some triangle's det
+// can reach Epsilon.
 __device__ __forceinline__ bool wide_begin(WideRay& r, WideState& s, WideHit& h, const WideView& w, const f3& pos,
                                            const f3& dir, float tmax) {
     wide_ray(r, pos, dir);
@@ -351,7 +362,7 @@ __device__ __forceinline__ bool wide_begin(WideRay& r, WideState& s, WideHit& h,
     if (!(w.nodes != 0u && tmax > kEpsilon && z == 0.0f)) return false;
     const float len = longest(dir);
     if (len >= kShortDir) return true;
-    if (len > 0.0f) h.best = kWalkRay;
+    if (len * w.reach >= kEpsilon) h.best = kWalkRay;
     return false;
 }
 

@@ -193,6 +193,7 @@ SceneView scene_view(const aur_scene* sc) {
     v.wide = sc->nmh->wide;
     v.nodes = sc->nmh->nodes;
     v.levels = sc->nmh->levels;
+    v.reach = wide_reach(sc->nmh);
     v.perm = sc->nmh->perm;
     v.normals = sc->normals;
     v.sids = sc->shader_ids;

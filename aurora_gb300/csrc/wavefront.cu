@@ -75,6 +75,7 @@ struct WfScene {
     uint32_t nodes;
     uint32_t levels;
     const uint4* wide;   // treelet records
+    float reach;         // WideView::reach
     float packet_span, dir_span;   // largest origin and direction spread of a warp packet
     uint32_t num_lights;
     uint32_t width, height;
@@ -165,7 +166,7 @@ __device__ __forceinline__ uint32_t agg_inc(uint32_t* ctr) {
 }
 
 __device__ __forceinline__ WideView scene_tree(const WfScene& sc) {
-    return WideView{sc.recs, sc.wide, sc.perm, sc.verts, sc.nodes, sc.levels};
+    return WideView{sc.recs, sc.wide, sc.perm, sc.verts, sc.nodes, sc.levels, sc.reach};
 }
 
 // The trees of a warp whose lanes' rays run in different scenes.
@@ -406,6 +407,7 @@ __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_extend(WfArgs a) {
                     w.wide = sc.wide;
                     w.nodes = sc.nodes;
                     w.levels = sc.levels;
+                    w.reach = sc.reach;
                     sw.scene[lane] = scene;
                     const float4 o = a.o[slot], d = a.d[slot];
                     WideHit h;
@@ -700,6 +702,7 @@ __global__ void __launch_bounds__(kWfMaxBlock, 4) k_wf_shadow(WfArgs a) {
                     w.wide = sc.wide;
                     w.nodes = sc.nodes;
                     w.levels = sc.levels;
+                    w.reach = sc.reach;
                     sw.scene[lane] = scene;
                     WideHit h;
                     running = wide_begin(r, s, h, w, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w);
@@ -1096,6 +1099,7 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
         w.mis_count = sc->mis_count;
         w.nodes = sc->nmh->nodes;
         w.levels = sc->nmh->levels;
+        w.reach = wide_reach(sc->nmh);
         w.wide = sc->nmh->wide;
         w.packet_span = packet_span(sc->nmh);
         w.dir_span = dir_span(sc->nmh);
