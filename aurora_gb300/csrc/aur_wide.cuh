@@ -519,8 +519,9 @@ __device__ __forceinline__ bool wide_step(const WideView& w, const WideRay& r, W
 //   first occluder: position in the ray's own test order
 // found so far. Rays go on to further treelets while their pairs wait, so a
 // box is now and then tested against a t that is about to shrink; what is
-// found is the same.
-#ifdef __CUDACC__
+// found is the same. (AUR_HOST_WARP: host builds that bring the warp
+// intrinsics along.)
+#if defined(__CUDACC__) || defined(AUR_HOST_WARP)
 struct WideQueue {
     float4 pd[32];                // pos.xyz, dir.x of each lane's ray
     float2 d[32];                 // dir.yz
@@ -589,7 +590,11 @@ __device__ __forceinline__ void queue_add(WideQueue& q, uint32_t lane, uint32_t&
         if (have == 0u) break;
         if (tris) {
             uint32_t lt;
+#ifdef __CUDACC__
             asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+#else
+            lt = (1u << lane) - 1u;
+#endif
             const uint32_t e = count + __popc(have & lt);
             q.idx[e] = wide_tri_index<kMode>(r, s, __ffs(tris) - 1);
             q.lane[e] = (uint8_t)lane;
@@ -632,7 +637,7 @@ __device__ __forceinline__ void wide_warp(const WideView& w, WideQueue& q, bool 
     h.t2 = __uint_as_float(q.t2[lane]);
     h.best = q.best[lane];
 }
-#endif  // __CUDACC__
+#endif  // __CUDACC__ || AUR_HOST_WARP
 
 // ------------------------------------------------------------ a few triangles
 // An NMH of at most kTinyTris triangles has no use for a tree: every lane
@@ -928,7 +933,7 @@ __device__ __forceinline__ uint32_t finish_any(const WideView& w, const WideRay&
 // each lane meets its triangles in its own order and its result is its own
 // walk's (in any hit, the first accepted triangle). Call with all 32 lanes;
 // `valid`: the lane has a ray; oct: the octant (dir_octant of any of them).
-#ifdef __CUDACC__
+#if defined(__CUDACC__) || defined(AUR_HOST_WARP)
 __device__ __forceinline__ float warp_min(float v) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -1034,6 +1039,6 @@ __device__ __forceinline__ void wide_packet(const WideView& w, bool valid, uint3
         if (!wide_next<kMode>(r, s)) break;
     }
 }
-#endif  // __CUDACC__
+#endif  // __CUDACC__ || AUR_HOST_WARP
 
 }  // namespace aur
