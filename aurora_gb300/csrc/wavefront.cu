@@ -23,6 +23,9 @@
 //   shade     : BSDF, light samples -> shadow-ray queue, the next ray -> queue
 // Batches with specular shaders take extend, shade, shadow and combine in this
 // order: the next ray comes from the path's stack once its colour is updated.
+// So do batches whose caller limits the iterations: combining one iteration
+// later takes one more iteration per wave, and hands slots back later, so that
+// a limit that suffices for this order would not.
 // Samples are processed in waves of `samples_per_wave` per pixel; a wave's
 // samples are added to each frame in sample order afterwards, as drawPixels
 // would. The whole render is one CUDA graph: an outer conditional while node
@@ -134,6 +137,7 @@ struct WfArgs {
     // component k (pos + weight, dir + eta, thr + pdf) at stk[(e * 3 + k) * Q + slot]
     float4* stk;
     uint32_t* sp;   // stack depth per slot
+    bool overlap;   // an iteration's shadow rays and combine belong to the next one
     cudaGraphConditionalHandle h_inner, h_outer;
     uint32_t in_graph;   // 1 when launched by the graph: only then may kernels set its conditionals
 };
@@ -144,14 +148,14 @@ __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 constexpr float kPathMissed = -1.0f, kPathEnds = 0.0f, kPathGoesOn = 1.0f;
 
 // Queues of an iteration: the paths it extends and shades, those it hands on,
-// and the previous iteration's. Batches without specular shaders trace an
-// iteration's shadow rays, and combine their paths, in the next one (see the
-// graph), whose extend stage does not depend on them.
+// and the previous iteration's. With `overlap` an iteration's shadow rays are
+// traced, and its paths combined, in the next one (see the graph), whose extend
+// stage does not depend on them.
 __device__ __forceinline__ uint32_t queue_cur(const WfCtl* c) { return c->iter % 3u; }
 __device__ __forceinline__ uint32_t queue_next(const WfCtl* c) { return (c->iter + 1u) % 3u; }
 __device__ __forceinline__ uint32_t queue_prev(const WfCtl* c) { return (c->iter + 2u) % 3u; }
 // The shadow rays a launch of the shadow stage traces.
-__device__ __forceinline__ uint32_t shadow_slot(const WfArgs& a) { return (a.ctl->iter + (a.stk ? 0u : 1u)) & 1u; }
+__device__ __forceinline__ uint32_t shadow_slot(const WfArgs& a) { return (a.ctl->iter + (a.overlap ? 1u : 0u)) & 1u; }
 
 // Warp-aggregated atomic increment.
 __device__ __forceinline__ uint32_t agg_inc(uint32_t* ctr) {
@@ -747,7 +751,7 @@ template <bool kMis, bool kSpec>
 __global__ void k_wf_combine(WfArgs a) {
     WfCtl* c = a.ctl;
     const uint32_t cur = queue_cur(c), nxt = queue_next(c);
-    const uint32_t from_q = kSpec ? cur : queue_prev(c);
+    const uint32_t from_q = !kSpec && a.overlap ? queue_prev(c) : cur;
     const uint32_t n = c->ext_count[from_q];
     for (uint32_t i = global_tid(); i < n; i += grid_threads()) {
         const uint32_t slot = a.ext_q[from_q][i];
@@ -824,14 +828,13 @@ __global__ void k_wf_combine(WfArgs a) {
 __global__ void k_wf_end(WfArgs a) {
     WfCtl* c = a.ctl;
     const uint32_t cur = queue_cur(c), nxt = queue_next(c);
-    const bool spec = a.stk != nullptr;
     c->total_ext += c->ext_count[cur];
     c->total_shadow += c->shadow_count[c->iter & 1u];
     c->shadow_count[shadow_slot(a)] = 0;
-    c->ext_count[spec ? cur : queue_prev(c)] = 0;
+    c->ext_count[a.overlap ? queue_prev(c) : cur] = 0;
     c->iter += 1;
     c->total_iters += 1;
-    // paths to extend, or (without specular shaders) to combine
+    // paths to extend, or (with overlap) to combine
     bool more = c->items_issued < c->items_total || c->ext_count[nxt] > 0 || c->ext_count[cur] > 0;
     if (c->iter > c->iter_limit) { c->error |= 1u; more = false; }
     if (c->error) more = false;
@@ -963,7 +966,7 @@ aur_status make_graph(aur_batch* bt) {
     AUR_CUDA(cudaStreamBeginCaptureToGraph(s, iter_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     k_wf_generate<<<g, bs, 0, s>>>(a);
     k_wf_generate_commit<<<1, 1, 0, s>>>(a);
-    if (a.stk) {
+    if (!a.overlap) {
         launch_extend(bt, a, s);
         launch_shade(a, g, bs, s);
         launch_shadow(bt, a, s);
@@ -1194,6 +1197,7 @@ aur_status aur_batch_create(aur_ctx* ctx, const aur_scene* const* scenes, const 
     a.defer = (uint32_t*)(base + o_def);
     a.stk = spec ? (float4*)(base + o_stk) : nullptr;
     a.sp = spec ? (uint32_t*)(base + o_sp) : nullptr;
+    a.overlap = !spec && tn.max_iterations == 0;
     cudaMemcpy(base + o_tab, table.data(), sizeof(WfScene) * num_scenes, cudaMemcpyHostToDevice);
     cudaMemcpy(base + o_pix, pix_off.data(), 4 * (num_scenes + 1), cudaMemcpyHostToDevice);
     WfCtl ctl{};
@@ -1321,7 +1325,6 @@ aur_status aur_batch_profile(aur_ctx* ctx, aur_batch* bt, float* const* accum, f
         stage_ms[stage] += ms;
     };
     const uint32_t g = bt->grid, bs = bt->block;
-    const bool spec = a.stk != nullptr;
     WfCtl c;
     AUR_CUDA(cudaMemcpyAsync(&c, a.ctl, sizeof(c), cudaMemcpyDeviceToHost, st));
     AUR_CUDA(cudaStreamSynchronize(st));
@@ -1337,19 +1340,19 @@ aur_status aur_batch_profile(aur_ctx* ctx, aur_batch* bt, float* const* accum, f
             cudaEventRecord(ev[1], st);
             launch_extend(bt, a, st);
             cudaEventRecord(ev[2], st);
-            if (spec) launch_shade(a, g, bs, st);
+            if (!a.overlap) launch_shade(a, g, bs, st);
             cudaEventRecord(ev[3], st);
             launch_shadow(bt, a, st);
             cudaEventRecord(ev[4], st);
             launch_combine(a, g, bs, st);
             cudaEventRecord(ev[5], st);
-            if (!spec) launch_shade(a, g, bs, st);
+            if (a.overlap) launch_shade(a, g, bs, st);
             cudaEventRecord(ev[6], st);
             k_wf_end<<<1, 1, 0, st>>>(a);
             AUR_CUDA(cudaMemcpyAsync(&c, a.ctl, sizeof(c), cudaMemcpyDeviceToHost, st));
             AUR_CUDA(cudaStreamSynchronize(st));
             lap(1, 0, 1); lap(2, 1, 2); lap(3, 2, 3); lap(4, 3, 4); lap(5, 4, 5); lap(3, 5, 6);
-            // c.iter is the next iteration: its queue, and the paths that the last one left to combine
+            // c.iter is the next iteration: its queue, and the paths that the last one left to combine (overlap)
             const bool more = (c.items_issued < c.items_total || c.ext_count[c.iter % 3u] > 0 ||
                                c.ext_count[(c.iter + 2u) % 3u] > 0) && !c.error;
             if (!more || it > c.iter_limit) break;
