@@ -265,7 +265,7 @@ aur_status aur_nmh_destroy(aur_nmh* nmh) {
     if (!nmh) return AUR_OK;
     cudaSetDevice(nmh->device);
     cudaDeviceSynchronize();   // no launch may still read it
-    if (nmh->mem && cudaFreeAsync(nmh->mem, cudaStreamLegacy) != cudaSuccess) cudaGetLastError();
+    if (nmh->mem) nmh->pool->release(nmh->mem);
     delete nmh;
     return AUR_OK;
 }

@@ -68,6 +68,9 @@ struct BuildCache;
 struct NmhPool {
     int device = 0;
     cudaMemPool_t pool = nullptr;
+    // Frees an NMH's memory that no launch uses any more. What the pool does
+    // not keep is the driver's again when this returns.
+    void release(void* mem);
     ~NmhPool();
 };
 

@@ -1598,10 +1598,19 @@ static float record_extent(const float* r, uint32_t nodes) {
 // NMH memory comes from a pool of the context, allocated and freed in stream
 // order: a plain cudaMalloc / cudaFree pair maps and unmaps device memory for
 // every NMH over 2 MB, which is most of a small rebuild's time. The pool keeps
-// at most kNmhPoolBytes of freed memory (a 1M-triangle NMH, rebuilt every
-// frame, takes 121 MB) and gives back what is above that at the next
-// synchronization, all of it with the context and its last NMH.
+// at most kNmhPoolBytes (a 1M-triangle NMH, rebuilt every frame, takes 121 MB)
+// and gives back what is above that when an NMH is destroyed, all of it with
+// the context and its last NMH.
 constexpr uint64_t kNmhPoolBytes = 256ull << 20;
+
+void NmhPool::release(void* mem) {
+    if (!mem) return;
+    if (cudaFreeAsync(mem, cudaStreamLegacy) != cudaSuccess) cudaGetLastError();
+    // a pool gives memory back when a stream is synchronized after the free
+    uint64_t held = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess || held > kNmhPoolBytes)
+        cudaStreamSynchronize(cudaStreamLegacy);
+}
 
 NmhPool::~NmhPool() {
     if (!pool) return;
@@ -1644,10 +1653,8 @@ aur_status nmh_build_impl(aur_ctx* ctx, const float* V, uint32_t count, aur_nmh*
 
     cudaStream_t st = ctx->stream;
     auto cleanup = [&]() {
-        if (nmh->mem) {
-            cudaStreamSynchronize(st);
-            cudaFreeAsync(nmh->mem, cudaStreamLegacy);
-        }
+        cudaStreamSynchronize(st);
+        nmh->pool->release(nmh->mem);
         delete nmh;
     };
     // records, treelet records, permutation and vertices in one allocation (records first: 128-byte aligned)
