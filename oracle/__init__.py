@@ -71,6 +71,17 @@ def lib():
     return _lib
 
 
+class ReferenceMissing(RuntimeError):
+    """The reference's sources, which a call compiles and runs, are not on this machine."""
+
+
+def _need_ref():
+    L = ref_lib()
+    if L is None:
+        raise ReferenceMissing("the reference sources are not on this machine")
+    return L
+
+
 def ref_lib():
     """The reference's own traversal compiled as host C++, or None."""
     global _ref
@@ -296,7 +307,7 @@ def render(nscene, params, camera=None, accum=None, nthreads=None, table=None):
 
 def ref_trace_closest(V_nmh, rays):
     """Reference intersect(): (t, u, v) float32 (n,3) and NMH position (n,)."""
-    L = ref_lib()
+    L = _need_ref()
     V = np.ascontiguousarray(V_nmh, np.float32); rays = np.ascontiguousarray(rays, T.ray_dtype)
     tuv = np.zeros((rays.shape[0], 3), np.float32); ids = np.zeros(rays.shape[0], np.int32)
     L.ref_trace_closest(_ptr(V), V.shape[0], _ptr(rays), rays.shape[0], _ptr(tuv), _ptr(ids))
@@ -312,7 +323,7 @@ def draw2(seed, scene, pixel, sample, ray, slot):
 
 def ref_uniform_order():
     """0 if the reference's area-light sample scales e1 by the first uniform drawn, 1 if by the second."""
-    return ref_lib().ref_uniform_order()
+    return _need_ref().ref_uniform_order()
 
 
 def ref_shade_hits(nscene, tangents, bitangents, rays8, tri, tuv, uniforms):
@@ -324,14 +335,14 @@ def ref_shade_hits(nscene, tangents, bitangents, rays8, tri, tuv, uniforms):
     tg, bt = np.ascontiguousarray(tangents, np.float32), np.ascontiguousarray(bitangents, np.float32)
     r8, tr, tv = (np.ascontiguousarray(rays8, np.float32), np.ascontiguousarray(tri, np.int32),
                   np.ascontiguousarray(tuv, np.float32))
-    ref_lib().ref_shade_hits(_ptr(nscene.V), _ptr(nscene.N), _ptr(tg), _ptr(bt), _ptr(nscene.S), nscene.V.shape[0],
-                             _ptr(nscene.shaders), nscene.shaders.shape[0], _ptr(nscene.lights),
-                             nscene.lights.shape[0], _ptr(r8), _ptr(tr), _ptr(tv), n, _ptr(u), u.shape[1], _ptr(out))
+    _need_ref().ref_shade_hits(_ptr(nscene.V), _ptr(nscene.N), _ptr(tg), _ptr(bt), _ptr(nscene.S), nscene.V.shape[0],
+                               _ptr(nscene.shaders), nscene.shaders.shape[0], _ptr(nscene.lights),
+                               nscene.lights.shape[0], _ptr(r8), _ptr(tr), _ptr(tv), n, _ptr(u), u.shape[1], _ptr(out))
     return out
 
 
 def ref_trace_any(V_nmh, rays):
-    L = ref_lib()
+    L = _need_ref()
     V = np.ascontiguousarray(V_nmh, np.float32); rays = np.ascontiguousarray(rays, T.ray_dtype)
     ids = np.zeros(rays.shape[0], np.int32)
     L.ref_trace_any(_ptr(V), V.shape[0], _ptr(rays), rays.shape[0], _ptr(ids))
@@ -369,8 +380,8 @@ def bsdf_hits(nscene, rays8, tri, tuv, uniforms, probes, tangents=None, bitangen
     args = [_ptr(keep[0]), _ptr(keep[1]), _ptr(keep[2]), n, _ptr(keep[3]), _ptr(keep[4]), _ptr(out)]
     if reference:
         tb = [np.ascontiguousarray(tangents, np.float32), np.ascontiguousarray(bitangents, np.float32)]
-        ref_lib().ref_bsdf_hits(_ptr(nscene.V), _ptr(nscene.N), _ptr(tb[0]), _ptr(tb[1]), _ptr(nscene.S),
-                                nscene.V.shape[0], _ptr(nscene.shaders), nscene.shaders.shape[0], *args)
+        _need_ref().ref_bsdf_hits(_ptr(nscene.V), _ptr(nscene.N), _ptr(tb[0]), _ptr(tb[1]), _ptr(nscene.S),
+                                  nscene.V.shape[0], _ptr(nscene.shaders), nscene.shaders.shape[0], *args)
     else:
         lib().orc_bsdf_hits(_ptr(nscene.V), _ptr(nscene.N), _ptr(nscene.S), nscene.V.shape[0], _ptr(nscene.shaders),
                             nscene.shaders.shape[0], *args[:-1], 1 if mis else 0, args[-1])
@@ -379,7 +390,7 @@ def bsdf_hits(nscene, rays8, tri, tuv, uniforms, probes, tangents=None, bitangen
 
 def mis_weight(a, b, reference=False):
     """The oracle's MIS weight 1 / (1 + (b/a)^2), or the reference's powerHeuristic(1, a, 1, b)."""
-    return (ref_lib().ref_power_heuristic if reference else lib().orc_mis_weight)(a, b)
+    return (_need_ref().ref_power_heuristic if reference else lib().orc_mis_weight)(a, b)
 
 
 def area_hit(light, pos, direction, reference=False):
@@ -389,7 +400,7 @@ def area_hit(light, pos, direction, reference=False):
     p = np.ascontiguousarray(pos, np.float32)           # held here: the call reads them through pointers
     d = np.ascontiguousarray(direction, np.float32)
     t = np.zeros(1, np.float32)
-    f = ref_lib().ref_area_hit if reference else lib().orc_hit_quad
+    f = _need_ref().ref_area_hit if reference else lib().orc_hit_quad
     h = f(_ptr(lt), _ptr(p), _ptr(d), _ptr(t))
     return bool(h), float(t[0])
 
@@ -412,5 +423,5 @@ def ref_triangle_areas(V):
     """Primitive3::area of each triangle (reference layout, (n, 9))."""
     V = np.ascontiguousarray(V, np.float32).reshape(-1, 9)
     out = np.zeros(V.shape[0], np.float32)
-    ref_lib().ref_triangle_areas(_ptr(V), V.shape[0], _ptr(out))
+    _need_ref().ref_triangle_areas(_ptr(V), V.shape[0], _ptr(out))
     return out
