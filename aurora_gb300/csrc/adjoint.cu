@@ -135,7 +135,7 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
                                           const f3& position, const f3& wo, float ew, bool bounce, uint32_t seed,
                                           uint32_t scene, uint32_t pixel, uint32_t sample, uint32_t rix, const f3& thr,
                                           const f3& g, float* __restrict__ d_light, f3& gl0, f3& Dp,
-                                          Grads& grads, uint32_t si, const Trav& trav, uint32_t* err) {
+                                          Grads& grads, uint32_t si, const Trav& trav) {
     f3 Li = kMis ? from(sh->emission_color) * ew : from(sh->emission_color);
     if (grads.emission) grads.add(true, si, kMis ? (g * thr) * ew : g * thr);
     Dp = mk3(0.0f);   // direct light per unit Lambert colour
@@ -152,8 +152,7 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
             f3 wdir; float wt, pdf;
             const f3 Ls = sample_light(L, position, seed, scene, pixel, sample, rix, 0u, wdir, wt, pdf);
             if (pdf > 0.0f && !zero(Ls)) {
-                if (!zero(f) &&
-                    !occluded(sc, trav, position, wdir, wt)) {
+                if (!zero(f) && !occluded(sc, trav, position, wdir, wt)) {
                     const float cs = fmaxf(0.0f, dot(wdir, b.N));
                     Li = Li + f * Ls * cs;
                     Dp = Dp + Ls * (kInvPi * cs);
@@ -199,8 +198,7 @@ __device__ __forceinline__ f3 direct_grad(const SceneView& sc, const aur_shader*
                 wpos.z += kEpsilon * wdir.z;
                 wt += kEpsilon;
                 if (lpdf > 0.0f && !zero(Lr)) {
-                        if (!zero(f) &&
-                        !occluded(sc, trav, wpos, wdir, wt)) {
+                    if (!zero(f) && !occluded(sc, trav, wpos, wdir, wt)) {
                         const float cs = fmaxf(0.0f, dot(wdir, b.N));
                         acc = acc + f * Lr * cs;
                         accp = accp + Lr * (kInvPi * cs);
@@ -303,7 +301,7 @@ __device__ void replay_stack(const SceneView& sc, uint32_t max_depth, uint32_t m
             continue_ray<kMis>(sh, b, cur, position, wo, path, depth, maxd, seed, scene, pixel, sample, rix);
         f3 Dp;
         const f3 Li = direct_grad<kMis>(sc, sh, b, f, position, wo, ew, bounce_follows, seed, scene, pixel, sample, rix,
-                                        cur.thr, g, d_light, gl0, Dp, grads, si, trav, err);
+                                        cur.thr, g, d_light, gl0, Dp, grads, si, trav);
         grads.add_diffuse(si, sh, g * (cur.thr * Dp));
         col = col + Li * cur.thr;
         for (int q = 0; q < kc.n; ++q) {
@@ -332,7 +330,7 @@ template <bool kMis, typename Trav, typename Grads>
 __device__ __forceinline__ void replay_diffuse(const SceneView& sc, uint32_t max_depth, uint32_t mode, uint32_t seed,
                                                uint32_t scene, uint32_t pixel, uint32_t sample, const PathRay& primary,
                                                const Trav& trav, const f3& g, Grads& grads,
-                                               float* __restrict__ d_light, f3& gl0, uint32_t* err) {
+                                               float* __restrict__ d_light, f3& gl0) {
     struct Marker {
         f3 col0, c1;          // colour before the subtree, the bouncing vertex's Lambert colour
         uint32_t si;
@@ -356,7 +354,7 @@ __device__ __forceinline__ void replay_diffuse(const SceneView& sc, uint32_t max
         const float ew = kMis ? emission_weight(sc, tri, dir, t, prev_pdf) : 1.0f;
         f3 Dp;
         const f3 Li = direct_grad<kMis>(sc, sh, b, f, position, wo, ew, nm + 1 <= max_depth, seed, scene, pixel, sample,
-                                        nm, thr, g, d_light, gl0, Dp, grads, si, trav, err);
+                                        nm, thr, g, d_light, gl0, Dp, grads, si, trav);
         grads.add_diffuse(si, sh, g * (thr * Dp));
         col = col + Li * thr;
         if (!path || nm + 1 > max_depth) break;
@@ -420,7 +418,7 @@ __global__ void __launch_bounds__(kAdjThreads, adj_blocks(kGeneric, kFew)) k_adj
         if constexpr (kGeneric)
             replay_stack<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, grads, dl, gl0, err);
         else
-            replay_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, grads, dl, gl0, err);
+            replay_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, g, grads, dl, gl0);
     }
     if constexpr (kFew) {      // the block's sums, one atomic per entry
         __shared__ float s_sum[kAdjThreads / 32][6 * kFewShaders];

@@ -527,7 +527,7 @@ template <typename Trav>
 __device__ __forceinline__ f3 direct_light_mis(const SceneView& sc, const aur_shader* sh, const Bsdf& b,
                                                const f3& position, const f3& wo, float ew, bool bounce,
                                                uint32_t seed, uint32_t scene, uint32_t pixel, uint32_t sample,
-                                               uint32_t rix, const Trav& trav, uint32_t* err) {
+                                               uint32_t rix, const Trav& trav) {
     f3 Li = from(sh->emission_color) * ew;
     const f3 f = bsdf_f(b);
     const uint32_t nl = sc.num_lights;
@@ -607,9 +607,9 @@ __device__ __forceinline__ f3 direct_light_mis(const SceneView& sc, const aur_sh
 template <bool kMis, typename Trav>
 __device__ __forceinline__ f3 direct_light(const SceneView& sc, const aur_shader* sh, const Bsdf& b, const f3& position,
                                            const f3& wo, float ew, bool bounce, uint32_t seed, uint32_t scene,
-                                           uint32_t pixel, uint32_t sample, uint32_t rix, const Trav& trav, uint32_t* err) {
+                                           uint32_t pixel, uint32_t sample, uint32_t rix, const Trav& trav) {
     if constexpr (kMis)
-        return direct_light_mis(sc, sh, b, position, wo, ew, bounce, seed, scene, pixel, sample, rix, trav, err);
+        return direct_light_mis(sc, sh, b, position, wo, ew, bounce, seed, scene, pixel, sample, rix, trav);
     f3 Li = from(sh->emission_color);
     for (uint32_t i = 0; i < sc.num_lights; ++i) {
         const aur_light& L = sc.lights[i];
@@ -776,7 +776,7 @@ __device__ __forceinline__ SampleResult integrate(const SceneView& sc, uint32_t 
         const bool specular = refl > 0.0f || trans > 0.0f;
         const float ew = kMis ? emission_weight(sc, tri, ray.dir, t, ray.pdf) : 1.0f;
         const f3 Li = direct_light<kMis>(sc, sh, b, position, wo, ew, !specular && depth + 1 <= maxd, seed, scene,
-                                         pixel, sample, rix, trav, err);
+                                         pixel, sample, rix, trav);
         const Continuation k =
             continue_ray<kMis>(sh, b, ray, position, wo, path, depth, maxd, seed, scene, pixel, sample, rix);
         for (int q = 0; q < k.n; ++q) {
@@ -793,7 +793,7 @@ __device__ __forceinline__ SampleResult integrate(const SceneView& sc, uint32_t 
 template <bool kMis, typename Trav>
 __device__ __forceinline__ SampleResult integrate_diffuse(const SceneView& sc, uint32_t max_depth, uint32_t mode,
                                                           uint32_t seed, uint32_t scene, uint32_t pixel,
-                                                          uint32_t sample, const PathRay& primary, const Trav& trav, uint32_t* err) {
+                                                          uint32_t sample, const PathRay& primary, const Trav& trav) {
     SampleResult res;
     res.color = mk3(0.0f);
     res.any_hit = false;
@@ -817,7 +817,7 @@ __device__ __forceinline__ SampleResult integrate_diffuse(const SceneView& sc, u
         const Bsdf b = get_bsdf(sc, sh, tri, u, v);
         const float ew = kMis ? emission_weight(sc, tri, dir, t, prev_pdf) : 1.0f;
         const f3 Li = direct_light<kMis>(sc, sh, b, position, wo, ew, depth + 1 <= max_depth, seed, scene, pixel,
-                                         sample, rix, trav, err);
+                                         sample, rix, trav);
         res.color = res.color + Li * thr;
         if (!path) break;
         if (++depth > max_depth) break;

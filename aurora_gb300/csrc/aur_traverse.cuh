@@ -272,8 +272,7 @@ template <bool kAny>
 __device__ __forceinline__ uint32_t traverse(const float4* __restrict__ recs, uint32_t nodes,
                                              const uint32_t* __restrict__ perm, const f3& pos, const f3& dir,
                                              float& best_t, float& bu, float& bv, const StackRef& stk,
-                                             uint32_t& visits, uint32_t* __restrict__ err) {
-    (void)err;
+                                             uint32_t& visits) {
     uint32_t best = kNoPrim;
     const f3 inv = box_inv(dir);
     TravState s;

@@ -852,7 +852,7 @@ static __device__ __forceinline__ float4 exact_walk(const float4* recs, uint32_t
     stk.cap = kStackDepth;
     float t = tmax, u = 0.0f, v = 0.0f;
     uint32_t visits = 0;
-    const uint32_t best = traverse<kAny>(recs, nodes, perm, mk3(px, py, pz), mk3(dx, dy, dz), t, u, v, stk, visits, nullptr);
+    const uint32_t best = traverse<kAny>(recs, nodes, perm, mk3(px, py, pz), mk3(dx, dy, dz), t, u, v, stk, visits);
     return make_float4(t, u, v, __uint_as_float(best));
 }
 

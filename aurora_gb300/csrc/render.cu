@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kRenderThreads, render_blocks(kMis, kTiny))
     const PathRay r = camera_ray(cam, p.width, p.height, pix % p.width, pix / p.width, s, p.spp);
     const SampleResult res =
         kGeneric ? integrate<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, err)
-                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav, err);
+                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, pix, s, r, trav);
     colors[t] = make_float4(res.color.x, res.color.y, res.color.z, res.any_hit ? 1.0f : 0.0f);
 }
 
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kRenderThreads) k_raytrace_mc(SceneView sc, au
     r.pdf = 0.0f;
     const SampleResult res =
         kGeneric ? integrate<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, id, sample, r, trav, err)
-                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, id, sample, r, trav, err);
+                 : integrate_diffuse<kMis>(sc, p.max_depth, p.mode, p.seed, p.scene_id, id, sample, r, trav);
     aur_hitpoint h = hits[id];
     h.color = to(from(h.color) + res.color);
     if (res.any_hit) {
