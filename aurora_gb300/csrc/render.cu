@@ -20,17 +20,18 @@ namespace aur {
 namespace {
 
 constexpr int kRenderThreads = 128;
-// Resident blocks per SM that the fused sample kernel is compiled for,
-// measured among 4 to 16. Trees: path mode 1.74 ms at 6 and 7, 1.75 at 8, 1.77 at
-// 9, 1.82 at 10 (200k-triangle spheres), 13.1, 13.7, 13.0, 13.2 and 14.0 ms (200k-
-// triangle terrain); the MIS estimator 2.41 ms at 6 to 8, 2.35 at 14
-// (4130-triangle box; its lanes diverge, and more warps to switch between pay
-// for the spills). Tiny scenes: 0.85 ms at 5, 6 and 8, 0.87 at 7, 0.88 at 9
-// (256x256 box, 16 samples); the MIS estimator 1.14 at 5 and 7, 1.18 at 8 and
-// 14 (301x233 emissive box, 9 samples). The per-tile kernel (k_raytrace_mc)
-// runs grids of one 65,536-ray tile, too small for occupancy to matter, and is
-// left unconstrained (a cap made it slower).
-constexpr int render_blocks(bool mis, bool tiny) { return tiny ? 7 : (mis ? 14 : 8); }
+// Resident blocks per SM that the fused sample kernel is compiled for. Trees,
+// path mode: 1.74 ms at 6 and 7, 1.75 at 8, 1.77 at 9, 1.82 at 10 (200k-triangle
+// spheres), 13.1, 13.7, 13.0, 13.2 and 14.0 ms (200k-triangle terrain); the MIS
+// estimator at 8, 12 and 14: 2.72, 3.01 and 3.40 ms (the spheres, 512x512, 4
+// samples), 12.9, 13.9 and 16.7 ms (the terrain, 480x270, 2 samples), 4.40, 4.43
+// and 4.58 ms (4130-triangle box, 256x256, 16 samples): more warps cost more in
+// spills than they hide. Tiny scenes, path mode at 5, 6, 7 and 8: 0.709, 0.713,
+// 0.706 and 0.708 ms (256x256 box, 16 samples); the MIS estimator 0.99, 1.01,
+// 1.03 and 1.035 ms (301x233 emissive box with an area light, 9 samples). The
+// per-tile kernel (k_raytrace_mc) runs grids of one 65,536-ray tile, too small
+// for occupancy to matter, and is left unconstrained (a cap made it slower).
+constexpr int render_blocks(bool mis, bool tiny) { return tiny ? (mis ? 5 : 7) : 8; }
 
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
