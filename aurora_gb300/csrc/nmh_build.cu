@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(kThreads) k_partition(ListSet ls, uint32_t M, 
 // Once every node segment of a level holds at most kLocalMax triangles, one
 // block per node of that level finishes its whole subtree with the same
 // per-level steps (select, emit, split, partition) on shared-memory copies of
-// the three lists, instead of 8 launches per remaining level over the whole
+// the three lists, instead of 3 launches per remaining level over the whole
 // soup. Triangles get block-local ids (their position in the first list);
 // lists hold local ids, the global node_of array is reused as the pid ->
 // local id map while the block loads its segment.
@@ -1092,7 +1092,8 @@ uint32_t log2i(uint32_t x) {
 constexpr size_t lookback_bytes(size_t ntiles) { return 3 * ntiles * sizeof(unsigned long long) + 16; }
 
 // No fewer than the levels that run over the whole soup (local_level): the
-// segments of level lv hold at most N / 2^lv triangles.
+// largest segment of a level, a full subtree, holds at most twice the level's
+// average, so at most N / 2^(lv - 1) triangles on level lv.
 constexpr size_t max_global_levels(size_t N) {
     size_t lv = 0;
     while ((N >> lv) > kLocalMax) ++lv;
@@ -1105,8 +1106,9 @@ constexpr size_t max_global_levels(size_t N) {
 // stream, or records them as a linear chain of CUDA graph nodes, or replays
 // the same sequence against such a recording and writes into its
 // instantiated graph only the arguments that differ (another vertex array,
-// other output buffers: the next build of the same size). A build makes six
-// launches per global level plus 20 (74 at 1M triangles); recorded once and
+// other output buffers: the next build of the same size). A build is three
+// launches per global level plus 18, a memset among them, or 14 where the sort
+// takes no scan launches (45 at 1M triangles, 26 at 20k); recorded once and
 // then launched as one graph they no longer wait on the host's per-launch
 // cost.
 struct NodeRec {

@@ -532,7 +532,8 @@ typedef struct aur_wavefront_tuning {
     uint32_t paths_in_flight;   /* path pool size (queue capacity) */
     uint32_t samples_per_wave;  /* samples per pixel processed per wave */
     uint32_t block_size;        /* threads per block of the stage kernels: multiple of 32, at most 256 */
-    uint32_t blocks_per_sm;     /* persistent grid = SMs x blocks_per_sm */
+    uint32_t blocks_per_sm;     /* persistent grid = SMs x blocks_per_sm (0: 6, and as many as fit for the
+                                 * two one-ray-per-lane traversal stages) */
     uint32_t max_iterations;    /* device-side loop limit per wave (0 = derived from the work): a pool that
                                  * holds the whole wave needs max_depth + 1 (without specular shaders), a
                                  * smaller one more. A batch with a limit does not trace shadow rays beside
