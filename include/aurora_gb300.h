@@ -229,7 +229,8 @@ typedef struct aur_nmh aur_nmh;
  * Builds on one context are serialized on the GPU (each call also waits for
  * its own build before returning). The NMH's memory comes from a pool of the
  * context, which keeps up to 256 MiB of destroyed NMHs' memory for the next
- * build until the context and the last NMH built on it are gone. */
+ * build until the context and the last NMH built on it are gone (an NMH of
+ * more than that, from 2.2M triangles on, maps its memory on each build). */
 aur_status aur_nmh_build(aur_ctx* ctx, const float* vertices, uint32_t count, aur_nmh** out);
 /* Test hook for the bounded waits of the build (no counterpart in the
  * reference, whose build waits on nothing on the device). The build's split
