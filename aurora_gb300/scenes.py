@@ -363,8 +363,11 @@ def microbench_rays(n=1 << 24, seed=1, image=4096, tmax=1.0e6):
 def sphere_scene(seed, min_tris=1000, max_tris=500_000):
     """N ~ U{1..200} spheres, radius U[0.05, 0.3], centre U[0,1]^3, each a UV
     sphere with a log-uniform triangle count in [80, 5000]; the total is kept
-    within [min_tris, max_tris] by dropping or adding spheres. One area light
+    within [min_tris, max_tris] by dropping or adding spheres, at least one of
+    which stays (max_tris >= 80). One area light
     above the unit cube, camera looking at the cube from +z."""
+    if max_tris < 80:
+        raise ValueError("sphere_scene: max_tris must be at least 80, the smallest sphere's triangles")
     rng = np.random.default_rng(seed)
     ns = int(rng.integers(1, 201))
     parts, total = [], 0
@@ -376,7 +379,9 @@ def sphere_scene(seed, min_tris=1000, max_tris=500_000):
         stacks = max(2, int(round(math.sqrt(tri / 4.0))))
         slices = max(3, int(round(tri / (2.0 * stacks))))
         if total + 2 * slices * stacks > max_tris:
-            break
+            if parts:
+                break
+            continue      # too large to be the only one: draw another
         parts.append(_uv_sphere(c, r, slices, stacks))
         total += 2 * slices * stacks
         i += 1
