@@ -35,19 +35,29 @@ constexpr uint32_t kRecStride = 8;          // float4 per node record
 constexpr uint32_t kSkipBit = 0x80000000u;
 constexpr float kBoxNear = 0.9999f, kBoxFar = 1.0001f;
 
-// Largest component of a direction, and the length from which the box tests
-// can follow it: they clamp reciprocals, and of a vector as short as the clamp
-// nothing but its signs would be left. Shorter rays are walked without boxes.
-// (A unit direction is 1e12 times as long; one this short needs triangles of
-// 300 units a side to reach Moller-Trumbore's det >= 1e-7 at all.)
+// Largest magnitude of three components, NaN if one is.
+__device__ __forceinline__ float largest(const f3& v) {
+#ifdef __CUDACC__
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fabsf(v.x)), "f"(fabsf(v.y)), "f"(fabsf(v.z)));
+    return r;
+#else
+    return v.x == v.x && v.y == v.y && v.z == v.z ? fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)) : NAN;
+#endif
+}
+
+// The largest component from which the box tests can follow a direction: they
+// clamp reciprocals, and of a vector as short as the clamp nothing but its
+// signs would be left. Shorter rays are walked without boxes. (A unit
+// direction is 1e12 times as long; one this short needs triangles of 300
+// units a side to reach Moller-Trumbore's det >= 1e-7 at all.)
 constexpr float kShortDir = 1e-12f;
-__device__ __forceinline__ float longest(const f3& d) { return fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z)); }
 
 // Reciprocal direction for box tests; zero components become +-1e-30 so that
 // no 0 * inf product (NaN) can occur. A short direction's are NaN: box_hit()
 // then drops every axis and prunes nothing, and slab_div() divides.
 __device__ __forceinline__ f3 box_inv(const f3& d) {
-    if (longest(d) < kShortDir) return mk3(NAN, NAN, NAN);
+    if (largest(d) < kShortDir) return mk3(NAN, NAN, NAN);
     return mk3(1.0f / copysignf(fmaxf(fabsf(d.x), 1e-30f), d.x), 1.0f / copysignf(fmaxf(fabsf(d.y), 1e-30f), d.y),
                1.0f / copysignf(fmaxf(fabsf(d.z), 1e-30f), d.z));
 }

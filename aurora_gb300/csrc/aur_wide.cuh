@@ -326,7 +326,7 @@ __device__ __forceinline__ uint32_t wide_order(bool nx, bool ny, bool nz) {
 __device__ __forceinline__ void wide_ray(WideRay& r, const f3& pos, const f3& dir) {
     r.pos = pos;
     r.dir = dir;
-    const float least = fminf(1e-20f, 1e-12f * fmaxf(longest(dir), kShortDir));
+    const float least = fminf(1e-20f, 1e-12f * fmaxf(largest(dir), kShortDir));
     r.inv = mk3(wide_recip(dir.x, least), wide_recip(dir.y, least), wide_recip(dir.z, least));
     r.order = wide_order(dir.x < 0.0f, dir.y < 0.0f, dir.z < 0.0f);
 }
@@ -373,9 +373,8 @@ __device__ __forceinline__ bool wide_begin(WideRay& r, WideState& s, WideHit& h,
     wide_init(s, w.levels);
     h.t = h.t2 = tmax;
     h.best = kNoPrim;
-    const float z = ((pos.x * 0.0f + pos.y * 0.0f) + (pos.z * 0.0f + dir.x * 0.0f)) + (dir.y * 0.0f + dir.z * 0.0f);
-    if (!(w.nodes != 0u && tmax > kEpsilon && z == 0.0f)) return false;
-    const float len = longest(dir);
+    const float len = largest(dir);
+    if (!(w.nodes != 0u && tmax > kEpsilon && largest(pos) < INFINITY && len < INFINITY)) return false;
     if (len >= kShortDir) return true;
     if (len * w.reach >= kEpsilon) h.best = kWalkRay;
     return false;
